@@ -46,6 +46,10 @@ struct SolverRows {
     float4* masses;    // tangent-1 and tangent-2 effective masses, depth, target speed
     float4* tangent1;  // [cap] tangent 1, twist mass
     float4* tangent2;  // [cap] tangent 2, 0
+    // the position pass's terms, once per step ([cap] each; write_position_terms)
+    float4* pnormal;  // normal, point count (0: no correction) | rows the contact owns << 4
+    uint4* prows;     // first row, second row, their inverse masses (bits; 0 for a row that is not moved)
+    float4* pdepth;   // the points' depths
 };
 
 // Control words (device-side counts the graph's kernels read instead of host values).
@@ -225,8 +229,7 @@ struct DeviceWorld {
     uint32_t* contributions;
     float4* resolution;
     // the position pass with its apply folded into the next iteration (worlds without joints)
-    int4* pd3;              // [3][n_cap] rotating linear position deltas (x, y, z, 0)
-    uint32_t* cnt3;         // [3][n_cap] rotating contribution counts
+    int4* pd3;              // [3][n_cap] rotating linear position deltas and contribution count (x, y, z, count)
     float4* resolution_alt; // [n_cap] the resolution of odd iterations
     uint32_t* cowner;       // [c_cap] bit 0 / bit 1: the contact claimed its first / second row
     // constraints (ball joints) and their solve order

@@ -1673,56 +1673,94 @@ __device__ __forceinline__ float coupling(const DBody& a, const DBody& b, f3 uj,
 }
 __device__ __forceinline__ void guard_row_masses(const BlockBodies& b, f3 normal, const f3* ra, const f3* rb, uint32_t pc,
                                                  float count_f, float* nm) {
+    // every loop runs over the four point slots and skips the unused ones, so that the arrays are
+    // indexed by constants and live in registers
     f3 u[4], v[4], iu[4], iv[4];
-    for (uint32_t j = 0; j < pc; ++j) {
+    bool converges = true;
+#pragma unroll
+    for (uint32_t j = 0; j < 4u; ++j) if (j < pc) {
         u[j] = cross(ra[j], normal);
         v[j] = cross(rb[j], normal);
         iu[j] = dbody_iinv(b.sf, u[j]);
         iv[j] = dbody_iinv(b.ss, v[j]);
+        converges = converges && nm[j] > 0.0f;
     }
-    bool converges = true;
-    for (uint32_t j = 0; j < pc; ++j) converges = converges && nm[j] > 0.0f;
     if (converges) {
-        // M = bound I - S, factored M = L diag(d) L^T row by row
+        // M = bound I - S, factored M = L diag(d) L^T row by row (the lower triangle is all it reads)
         float m[4][4], l[4][4], d[4];
-        for (uint32_t j = 0; j < pc; ++j)
-            for (uint32_t k = 0; k < pc; ++k)
+#pragma unroll
+        for (uint32_t j = 0; j < 4u; ++j)
+#pragma unroll
+            for (uint32_t k = 0; k <= j; ++k) if (j < pc)
                 m[j][k] = (j == k ? kRowMassBound : 0.0f) - coupling(b.sf, b.ss, u[j], v[j], iu[k], iv[k]) / sqrtf(nm[j] * nm[k]);
-        for (uint32_t j = 0; j < pc && converges; ++j) {
+#pragma unroll
+        for (uint32_t j = 0; j < 4u; ++j) if (j < pc && converges) {
             float pivot = m[j][j];
+#pragma unroll
             for (uint32_t k = 0; k < j; ++k) pivot = pivot - l[j][k] * l[j][k] * d[k];
             d[j] = pivot;
             converges = pivot > 0.0f;
-            for (uint32_t i = j + 1; i < pc && converges; ++i) {
+#pragma unroll
+            for (uint32_t i = j + 1; i < 4u; ++i) if (i < pc && converges) {
                 float x = m[i][j];
+#pragma unroll
                 for (uint32_t k = 0; k < j; ++k) x = x - l[i][k] * l[j][k] * d[k];
                 l[i][j] = x / pivot;
             }
         }
     }
     if (converges) return;
-    for (uint32_t j = 0; j < pc; ++j) nm[j] = count_f * coupling(b.sf, b.ss, u[j], v[j], iu[j], iv[j]);
+#pragma unroll
+    for (uint32_t j = 0; j < 4u; ++j) if (j < pc) nm[j] = count_f * coupling(b.sf, b.ss, u[j], v[j], iu[j], iv[j]);
 }
 
-__global__ void k_solve_prepare(DeviceWorld w) {
+// What the position pass asks of a contact, in three float4 columns that it streams (48 bytes for a
+// contact instead of 68 and four 32-byte body sectors): the normal with the point count (0: nothing
+// to correct) and the rows the contact owns, the two rows with their inverse masses (0 for a row
+// that does not move), the points' depths. None of it changes while a step's substeps run.
+__device__ __forceinline__ void write_position_terms(const DeviceWorld& w, uint32_t i, uint4 r, const BlockBodies& b) {
+    const uint32_t cap = w.c_cap;
+    const uint32_t pc = r.z & 0xFFu;
+    float depth[4];
+#pragma unroll
+    for (uint32_t pi = 0; pi < 4u; ++pi) depth[pi] = pi < pc ? w.cur.la[(size_t)pi * cap + i].w : 0.0f;
+    const uint32_t points = w.cur.mat[i].z > 0.0f ? 0u : pc;  // a soft contact is left to the velocity pass
+    const float ima = dbody_inert(b.pf) ? 0.0f : b.pf.inverse_mass;
+    const float imb = dbody_inert(b.ps) ? 0.0f : b.ps.inverse_mass;
+    w.srows.pnormal[i] = mk4(xyz(w.cur.normal[i]), __uint_as_float(points | (w.cowner[i] << 4)));
+    w.srows.prows[i] = make_uint4(r.x, r.y, __float_as_uint(ima), __float_as_uint(imb));
+    w.srows.pdepth[i] = make_float4(depth[0], depth[1], depth[2], depth[3]);
+}
+
+__global__ void __launch_bounds__(256) k_solve_prepare(DeviceWorld w, bool position_terms) {
     const uint32_t count = w.ctl[CTL_CONTACTS];
     const uint32_t cap = w.c_cap;
     const SolverRows& sr = w.srows;
     GRID_STRIDE(i, count) {
         uint4 r = w.cur.rows[i];
-        if (!resolves(r)) continue;
+        if (!resolves(r)) {
+            if (position_terms) sr.pnormal[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            continue;
+        }
         const BlockBodies b = block_bodies(w, r);
+        if (position_terms) write_position_terms(w, i, r, b);
         if (dbody_inert(b.pf) && dbody_inert(b.ps)) continue;
         f3 normal = xyz(w.cur.normal[i]);
+        const uint32_t pc = r.z & 0xFFu;
+        float4 la[4], lb[4];
+#pragma unroll
+        for (uint32_t pi = 0; pi < 4u; ++pi) if (pi < pc) {
+            la[pi] = w.cur.la[(size_t)pi * cap + i];
+            lb[pi] = w.cur.lb[(size_t)pi * cap + i];
+        }
         f3 t1, t2;
         make_tangents(normal, &t1, &t2);
-        uint32_t pc = r.z & 0xFFu;
         f3 ra[4], rb[4];
         f3 reach_f = s3(0.0f), reach_s = s3(0.0f);
-        for (uint32_t pi = 0; pi < pc; ++pi) {
-            size_t o = (size_t)pi * cap + i;
-            f3 af = arm(b.pf, xyz(w.cur.la[o]));
-            f3 as = arm(b.ps, xyz(w.cur.lb[o]));
+#pragma unroll
+        for (uint32_t pi = 0; pi < 4u; ++pi) if (pi < pc) {
+            f3 af = arm(b.pf, xyz(la[pi]));
+            f3 as = arm(b.ps, xyz(lb[pi]));
             ra[pi] = af - dbody_com(b.pf);
             rb[pi] = as - dbody_com(b.ps);
             reach_f = reach_f + ra[pi];
@@ -1732,13 +1770,15 @@ __global__ void k_solve_prepare(DeviceWorld w) {
         f3 spread_f = dbody_iinv(b.sf, cross(reach_f, normal));
         f3 spread_s = dbody_iinv(b.ss, cross(reach_s, normal));
         float nm[4];
-        for (uint32_t pi = 0; pi < pc; ++pi) {
+#pragma unroll
+        for (uint32_t pi = 0; pi < 4u; ++pi) if (pi < pc) {
             f3 arm_f = cross(ra[pi], normal);
             f3 arm_s = cross(rb[pi], normal);
             nm[pi] = count_f * (b.sf.inverse_mass + b.ss.inverse_mass) + dot(spread_f, arm_f) + dot(spread_s, arm_s);
         }
         if ((w.solver_guard & DYN_SOLVER_GUARD_ROW_MASS) && pc >= 2u) guard_row_masses(b, normal, ra, rb, pc, count_f, nm);
-        for (uint32_t pi = 0; pi < pc; ++pi) {
+#pragma unroll
+        for (uint32_t pi = 0; pi < 4u; ++pi) if (pi < pc) {
             size_t o = (size_t)pi * cap + i;
             float normal_mass = nm[pi];
             float truth = momentum_mass_arms(b.pf, b.ps, ra[pi], rb[pi], normal);
@@ -1746,7 +1786,7 @@ __global__ void k_solve_prepare(DeviceWorld w) {
             float t2_mass = momentum_mass_arms(b.sf, b.ss, ra[pi], rb[pi], t2) * count_f;
             sr.arm_a[o] = mk4(ra[pi], normal_mass);
             sr.arm_b[o] = mk4(rb[pi], truth);
-            sr.masses[o] = make_float4(t1_mass, t2_mass, w.cur.la[o].w, w.cur.lb[o].w);
+            sr.masses[o] = make_float4(t1_mass, t2_mass, la[pi].w, lb[pi].w);
         }
         float twist_mass = dot(normal, dbody_iinv(b.sf, normal)) + dot(normal, dbody_iinv(b.ss, normal));
         sr.tangent1[i] = mk4(t1, twist_mass);
@@ -1769,11 +1809,19 @@ __global__ void k_warm(DeviceWorld w) {
         f3 normal = xyz(w.cur.normal[i]);
         f3 t1 = xyz(sr.tangent1[i]), t2 = xyz(sr.tangent2[i]);
         uint32_t pc = r.z & 0xFFu;
-        for (uint32_t pi = 0; pi < pc; ++pi) {
+        // every point's loads before the first impulse
+        float4 acc[4], a4[4], b4[4];
+#pragma unroll
+        for (uint32_t pi = 0; pi < 4u; ++pi) if (pi < pc) {
             size_t o = (size_t)pi * cap + i;
-            float4 acc = w.cur.acc[o];
-            f3 j = normal * acc.x + t1 * acc.y + t2 * acc.z;
-            pair_impulse_arms(&f, &s, xyz(sr.arm_a[o]), xyz(sr.arm_b[o]), j);
+            acc[pi] = w.cur.acc[o];
+            a4[pi] = sr.arm_a[o];
+            b4[pi] = sr.arm_b[o];
+        }
+#pragma unroll
+        for (uint32_t pi = 0; pi < 4u; ++pi) if (pi < pc) {
+            f3 j = normal * acc[pi].x + t1 * acc[pi].y + t2 * acc[pi].z;
+            pair_impulse_arms(&f, &s, xyz(a4[pi]), xyz(b4[pi]), j);
         }
         // an inert (frozen) body's delta is exactly zero: its atomics would add nothing
         if (!dbody_inert(fl))
@@ -1781,6 +1829,16 @@ __global__ void k_warm(DeviceWorld w) {
         if (!dbody_inert(sl))
             accumulate(w.vdelta, r.y, s.velocity - sl.velocity, s.angular_velocity - sl.angular_velocity, DYN_SOLVER_VELOCITY_SCALE);
     }
+}
+
+constexpr float kFiniteMax = 3.402823466e38f;
+// One point's terms of a block (slot o of the point columns). The pose-only terms do not change
+// while k_solve runs.
+struct BlockPoint {
+    float4 acc, arm_a, arm_b, masses;
+};
+__device__ __forceinline__ BlockPoint load_point(const DeviceWorld& w, size_t o) {
+    return BlockPoint{w.cur.acc[o], __ldg(w.srows.arm_a + o), __ldg(w.srows.arm_b + o), __ldg(w.srows.masses + o)};
 }
 
 // solver_contact_block.wgsl:6-193 (Jacobi block with mass splitting); the pose-only terms come
@@ -1820,16 +1878,20 @@ __device__ __forceinline__ void solve_block(const DeviceWorld& w, const dyn_step
     // One point at a time: every point's impulse is computed from the velocities the block started
     // with (pf, ps), so applying each to first/second as soon as it is known gives the same sums,
     // in the same order, as applying all four after the loop; the old normal accumulators are summed
-    // in point order as they are read. Only one point's data is live at a time.
+    // in point order as they are read. The next point's four loads are issued before the current
+    // point's arithmetic (the first two points' beside the bodies'), so a block waits for two round
+    // trips (its rows, then everything else) instead of one for every point.
     float normal_total = 0.0f;
+    BlockPoint at[2];
+    if (pc > 0u) at[0] = load_point(w, i);
+    if (pc > 1u) at[1] = load_point(w, (size_t)cap + i);
     #pragma unroll
     for (uint32_t pi = 0; pi < 4u; ++pi) if (pi < pc) {
         size_t o = (size_t)pi * cap + i;
-        float4 acc = w.cur.acc[o];
+        const float4 acc = at[pi & 1u].acc, a4 = at[pi & 1u].arm_a, b4 = at[pi & 1u].arm_b, m2 = at[pi & 1u].masses;
+        if (pi < 2u && pi + 2u < pc) at[pi & 1u] = load_point(w, o + 2u * (size_t)cap);
         if (tape_acc) tape_acc[(size_t)pi * w.tape.c + i] = acc;
         normal_total = normal_total + wmax(acc.x, 0.0f);
-        float4 a4 = sr.arm_a[o], b4 = sr.arm_b[o];
-        float4 m2 = sr.masses[o];
         const f3 ra = xyz(a4), rb = xyz(b4);
         float normal_mass = a4.w, truth = b4.w;
         float depth = m2.z, target = m2.w;
@@ -1866,7 +1928,10 @@ __device__ __forceinline__ void solve_block(const DeviceWorld& w, const dyn_step
     f3 rel_spin = second.angular_velocity - first.angular_velocity;
     f3 planar = rel_spin - normal * dot(rel_spin, normal);
     float planar_len = length(planar);
-    if (planar_len > 1e-6f) {
+    // Without rolling (spin) friction the limit is zero times a finite total and the applied impulse
+    // zero: the body torques below would add nothing, so finite blocks skip them.
+    const bool finite = planar_len <= kFiniteMax && normal_total <= kFiniteMax;
+    if (planar_len > 1e-6f && !(finite && mat.x == 0.0f)) {
         f3 axis = planar / planar_len;
         float mass = dot(axis, dbody_iinv(b.sf, axis)) + dot(axis, dbody_iinv(b.ss, axis));
         if (mass > 0.0f) {
@@ -1877,7 +1942,7 @@ __device__ __forceinline__ void solve_block(const DeviceWorld& w, const dyn_step
         }
     }
     float twist = dot(rel_spin, normal);
-    if (fabsf(twist) > 1e-6f) {
+    if (fabsf(twist) > 1e-6f && !(finite && fabsf(twist) <= kFiniteMax && mat.y == 0.0f)) {
         if (twist_mass > 0.0f) {
             float limit = mat.y * normal_total;
             float applied = wclamp(-twist / twist_mass, -limit, limit);
@@ -1903,27 +1968,28 @@ __global__ void __launch_bounds__(256, 2) k_solve(DeviceWorld w, dyn_step_params
     GRID_STRIDE(i, count) solve_block(w, p, i, residual, tape_index);
 }
 
-// solver_block_apply.wgsl:7-29
-__device__ __forceinline__ void apply_velocity_row(const DeviceWorld& w, uint32_t i) {
-    uint32_t row = w.solver_rows[i];
+// solver_block_apply.wgsl:7-29. Only a moving row's words are ever summed into (an inert row's delta
+// is zero), so the pass walks the dynamic rows themselves and stops at a row whose words are zero:
+// one load behind the row index instead of the chain through the solver row list, and no store to
+// a row that nothing touched.
+__device__ __forceinline__ void apply_velocity_row(const DeviceWorld& w, uint32_t row) {
     int4* d = reinterpret_cast<int4*>(w.vdelta + 8u * row);
     int4 a = d[0], b = d[1];
+    if ((a.x | a.y | a.z | a.w | b.x | b.y) == 0) return;
+    BodyHot& h = w.hot[row];
+    float4 v = h.vel, av = h.ang;
     d[0] = make_int4(0, 0, 0, 0);
     d[1] = make_int4(0, 0, 0, 0);
     f3 lin = mk3((float)a.x / DYN_SOLVER_VELOCITY_SCALE, (float)a.y / DYN_SOLVER_VELOCITY_SCALE,
                  (float)a.z / DYN_SOLVER_VELOCITY_SCALE);
     f3 ang = mk3((float)a.w / DYN_SOLVER_VELOCITY_SCALE, (float)b.x / DYN_SOLVER_VELOCITY_SCALE,
                  (float)b.y / DYN_SOLVER_VELOCITY_SCALE);
-    if (is_zero3(lin) && is_zero3(ang)) return;
-    BodyHot& h = w.hot[row];
-    float4 v = h.vel, av = h.ang;
     h.vel = make_float4(v.x + lin.x, v.y + lin.y, v.z + lin.z, v.w);
     h.ang = make_float4(av.x + ang.x, av.y + ang.y, av.z + ang.z, av.w);
 }
 __global__ void k_vapply(DeviceWorld w) {
-    const uint32_t rows = w.ctl[CTL_SOLVER_ROWS];
-    if (blockIdx.x == 0 && threadIdx.x == 0 && rows > 0u) w.ctl[CTL_ROUNDS] += 1u;
-    GRID_STRIDE(i, rows) apply_velocity_row(w, i);
+    if (blockIdx.x == 0 && threadIdx.x == 0 && w.ctl[CTL_SOLVER_ROWS] > 0u) w.ctl[CTL_ROUNDS] += 1u;
+    GRID_STRIDE(row, w.nd) apply_velocity_row(w, row);
 }
 
 // substep_integrate.wgsl:15-76 (no force fields)
@@ -1989,53 +2055,66 @@ __global__ void k_advance(DeviceWorld w, dyn_step_params p) {
     }
 }
 
-// position_correction.wgsl:5-46 with position_block.wgsl:11-33
-__device__ __forceinline__ void position_block(const DeviceWorld& w, const dyn_step_params& p, uint32_t i) {
-    const uint32_t cap = w.c_cap;
-    uint4 r = w.cur.rows[i];
-    if (!resolves(r)) return;
-    float4 mat = w.cur.mat[i];
-    if (mat.z > 0.0f) return;
-    const BodyHot& ha = w.hot[r.x];
-    const BodyHot& hb = w.hot[r.y];
-    float ima = (!simulates(ha.pos.w, ha.aux.y) || ha.aux.x != 0u) ? 0.0f : ha.pos.w;
-    float imb = (!simulates(hb.pos.w, hb.aux.y) || hb.aux.x != 0u) ? 0.0f : hb.pos.w;
-    f3 normal = xyz(w.cur.normal[i]);
-    float resolved = dot(normal, xyz(w.resolution[r.y]) - xyz(w.resolution[r.x]));
+// position_correction.wgsl:5-46 with position_block.wgsl:11-33, from the columns write_position_terms
+// left: the corrections of the two rows, or false when the contact contributes nothing.
+struct PositionTerms {
+    float4 normal;  // normal, point count | owned rows << 4
+    uint4 rows;     // the rows, their inverse masses
+    float4 depth;
+};
+__device__ __forceinline__ PositionTerms load_position_terms(const DeviceWorld& w, uint32_t i) {
+    return PositionTerms{__ldg(w.srows.pnormal + i), __ldg(w.srows.prows + i), __ldg(w.srows.pdepth + i)};
+}
+__device__ __forceinline__ uint32_t position_points(const PositionTerms& t) { return __float_as_uint(t.normal.w) & 15u; }
+__device__ __forceinline__ uint32_t position_owned(const PositionTerms& t) { return __float_as_uint(t.normal.w) >> 4; }
+__device__ __forceinline__ bool position_correction(const dyn_step_params& p, const PositionTerms& t, float4 res_a, float4 res_b,
+                                                    f3* la, f3* lb) {
+    const float ima = __uint_as_float(t.rows.z), imb = __uint_as_float(t.rows.w);
+    const f3 normal = xyz(t.normal);
+    const uint32_t pc = position_points(t);
+    float resolved = dot(normal, xyz(res_b) - xyz(res_a));
+    const float depth[4] = {t.depth.x, t.depth.y, t.depth.z, t.depth.w};
     f3 total = s3(0.0f);
     uint32_t contributing = 0;
-    uint32_t pc = r.z & 0xFFu;
-    for (uint32_t pi = 0; pi < pc; ++pi) {
-        float error = wmax(w.cur.la[(size_t)pi * cap + i].w - p.slop - resolved, 0.0f);
+    const float k = ima + imb;
+    if (k == 0.0f) return false;
+#pragma unroll
+    for (uint32_t pi = 0; pi < 4u; ++pi) if (pi < pc) {
+        float error = wmax(depth[pi] - p.slop - resolved, 0.0f);
         if (error <= 0.0f) continue;
-        float k = ima + imb;
-        if (k == 0.0f) continue;
         total = total + normal * (p.relaxation * error / k);
         contributing += 1;
     }
-    if (contributing == 0u) return;
+    if (contributing == 0u) return false;
     f3 correction = total / (float)contributing;
-    f3 la = -correction * ima;
-    f3 lb = correction * imb;
-    if (!(dot(la, la) > 0.0f || dot(lb, lb) > 0.0f)) return;
+    *la = -correction * ima;
+    *lb = correction * imb;
+    return dot(*la, *la) > 0.0f || dot(*lb, *lb) > 0.0f;
+}
+__device__ __forceinline__ void position_block(const DeviceWorld& w, const dyn_step_params& p, uint32_t i) {
+    const PositionTerms t = load_position_terms(w, i);
+    if (position_points(t) == 0u) return;
+    const uint32_t ra = t.rows.x, rb = t.rows.y;
+    f3 la, lb;
+    if (!position_correction(p, t, w.resolution[ra], w.resolution[rb], &la, &lb)) return;
     // Both rows are marked as contributing (position_apply renormalises a contributed row's
     // orientation). A moving row needs the exact count, which divides its summed delta; a
     // frozen row's sum is zero, so only "contributed" matters there: every writer stores the
     // same 1, without an atomic on the shared row of a static body.
-    if (ima > 0.0f) {
-        atomicAdd(&w.contributions[r.x], 1u);
-        accumulate_linear(w.pdelta, r.x, la, DYN_SOLVER_POSITION_SCALE);
-    } else if (w.contributions[r.x] == 0u) {
-        w.contributions[r.x] = 1u;
+    if (__uint_as_float(t.rows.z) > 0.0f) {
+        atomicAdd(&w.contributions[ra], 1u);
+        accumulate_linear(w.pdelta, ra, la, DYN_SOLVER_POSITION_SCALE);
+    } else if (w.contributions[ra] == 0u) {
+        w.contributions[ra] = 1u;
     }
-    if (imb > 0.0f) {
-        atomicAdd(&w.contributions[r.y], 1u);
-        accumulate_linear(w.pdelta, r.y, lb, DYN_SOLVER_POSITION_SCALE);
-    } else if (w.contributions[r.y] == 0u) {
-        w.contributions[r.y] = 1u;
+    if (__uint_as_float(t.rows.w) > 0.0f) {
+        atomicAdd(&w.contributions[rb], 1u);
+        accumulate_linear(w.pdelta, rb, lb, DYN_SOLVER_POSITION_SCALE);
+    } else if (w.contributions[rb] == 0u) {
+        w.contributions[rb] = 1u;
     }
 }
-__global__ void k_position(DeviceWorld w, dyn_step_params p) {
+__global__ void __launch_bounds__(256) k_position(DeviceWorld w, dyn_step_params p) {
     const uint32_t count = w.ctl[CTL_CONTACTS];
     GRID_STRIDE(i, count) position_block(w, p, i);
 }
@@ -2083,14 +2162,14 @@ struct RowCorrection {
     f3 al;
     uint32_t contributing;
 };
-__device__ __forceinline__ RowCorrection row_correction(const int4* __restrict__ pd, const uint32_t* __restrict__ cnt, uint32_t row) {
+// A row's words are one int4: the three deltas and the contribution count.
+__device__ __forceinline__ RowCorrection row_correction(int4 words) {
     RowCorrection c;
-    c.contributing = cnt[row];
+    c.contributing = (uint32_t)words.w;
     c.al = s3(0.0f);
     if (c.contributing != 0u) {
-        const int4 a = pd[row];
-        const f3 lin = mk3((float)a.x / DYN_SOLVER_POSITION_SCALE, (float)a.y / DYN_SOLVER_POSITION_SCALE,
-                           (float)a.z / DYN_SOLVER_POSITION_SCALE);
+        const f3 lin = mk3((float)words.x / DYN_SOLVER_POSITION_SCALE, (float)words.y / DYN_SOLVER_POSITION_SCALE,
+                           (float)words.z / DYN_SOLVER_POSITION_SCALE);
         c.al = lin / (float)c.contributing;
     }
     return c;
@@ -2100,61 +2179,25 @@ __device__ __forceinline__ float4 corrected(float4 res, const RowCorrection& c) 
     return make_float4(res.x + c.al.x, res.y + c.al.y, res.z + c.al.z, 0.0f);
 }
 // apply_position_row's pose update: a pure translation, and the orientation renormalised
-__device__ __forceinline__ void move_row(const DeviceWorld& w, uint32_t row, const RowCorrection& c) {
+__device__ __forceinline__ void move_row(const DeviceWorld& w, uint32_t row, const RowCorrection& c, float4 at, float4 turned) {
     if (c.contributing == 0u) return;
     const f3 aa = s3(0.0f) / (float)c.contributing;
     BodyHot& h = w.hot[row];
-    const f3 pos = xyz(h.pos) + c.al;
-    h.pos = mk4(pos, h.pos.w);
+    const f3 pos = xyz(at) + c.al;
     const f3 ha = aa * 0.5f;
-    h.rot = normalize4(quat_mul(make_float4(ha.x, ha.y, ha.z, 1.0f), h.rot));
+    h.pos = mk4(pos, at.w);
+    h.rot = normalize4(quat_mul(make_float4(ha.x, ha.y, ha.z, 1.0f), turned));
 }
-__device__ __forceinline__ void position_block_rows(const DeviceWorld& w, const dyn_step_params& p, uint32_t i, uint4 r,
-                                                    float4 res_a, float4 res_b, int4* __restrict__ pd,
-                                                    uint32_t* __restrict__ cnt) {
-    const uint32_t cap = w.c_cap;
-    if (!resolves(r)) return;
-    float4 mat = w.cur.mat[i];
-    if (mat.z > 0.0f) return;
-    const BodyHot& ha = w.hot[r.x];
-    const BodyHot& hb = w.hot[r.y];
-    float ima = (!simulates(ha.pos.w, ha.aux.y) || ha.aux.x != 0u) ? 0.0f : ha.pos.w;
-    float imb = (!simulates(hb.pos.w, hb.aux.y) || hb.aux.x != 0u) ? 0.0f : hb.pos.w;
-    f3 normal = xyz(w.cur.normal[i]);
-    float resolved = dot(normal, xyz(res_b) - xyz(res_a));
-    f3 total = s3(0.0f);
-    uint32_t contributing = 0;
-    uint32_t pc = r.z & 0xFFu;
-    for (uint32_t pi = 0; pi < pc; ++pi) {
-        float error = wmax(w.cur.la[(size_t)pi * cap + i].w - p.slop - resolved, 0.0f);
-        if (error <= 0.0f) continue;
-        float k = ima + imb;
-        if (k == 0.0f) continue;
-        total = total + normal * (p.relaxation * error / k);
-        contributing += 1;
-    }
-    if (contributing == 0u) return;
-    f3 correction = total / (float)contributing;
-    f3 la = -correction * ima;
-    f3 lb = correction * imb;
-    if (!(dot(la, la) > 0.0f || dot(lb, lb) > 0.0f)) return;
-    int32_t* da = reinterpret_cast<int32_t*>(pd + r.x);
-    int32_t* db = reinterpret_cast<int32_t*>(pd + r.y);
-    if (ima > 0.0f) {
-        atomicAdd(&cnt[r.x], 1u);
-        atomicAdd(da + 0, solver_word(la.x, DYN_SOLVER_POSITION_SCALE));
-        atomicAdd(da + 1, solver_word(la.y, DYN_SOLVER_POSITION_SCALE));
-        atomicAdd(da + 2, solver_word(la.z, DYN_SOLVER_POSITION_SCALE));
-    } else if (cnt[r.x] == 0u) {
-        cnt[r.x] = 1u;
-    }
-    if (imb > 0.0f) {
-        atomicAdd(&cnt[r.y], 1u);
-        atomicAdd(db + 0, solver_word(lb.x, DYN_SOLVER_POSITION_SCALE));
-        atomicAdd(db + 1, solver_word(lb.y, DYN_SOLVER_POSITION_SCALE));
-        atomicAdd(db + 2, solver_word(lb.z, DYN_SOLVER_POSITION_SCALE));
-    } else if (cnt[r.y] == 0u) {
-        cnt[r.y] = 1u;
+// A correction into a row's words of this iteration.
+__device__ __forceinline__ void contribute(int4* pd, uint32_t row, float inverse_mass, f3 linear) {
+    int32_t* d = reinterpret_cast<int32_t*>(pd + row);
+    if (inverse_mass > 0.0f) {
+        atomicAdd(d + 3, 1);
+        atomicAdd(d + 0, solver_word(linear.x, DYN_SOLVER_POSITION_SCALE));
+        atomicAdd(d + 1, solver_word(linear.y, DYN_SOLVER_POSITION_SCALE));
+        atomicAdd(d + 2, solver_word(linear.z, DYN_SOLVER_POSITION_SCALE));
+    } else if (d[3] == 0) {
+        d[3] = 1;  // a frozen row: only "contributed" matters (position_block)
     }
 }
 // A taped step's position snapshots, written by each solver row's owner: the resolution iteration
@@ -2166,53 +2209,66 @@ __device__ __forceinline__ void tape_position_row(const TapeWrites& t, uint32_t 
     t.res[(base + k) * t.n + row] = res;
     if (with_count) t.cnt[(base + k - 1u) * t.n + row] = count;
 }
+// Bound by the latency of its gathers (a few percent of the memory rate): the contact's three
+// columns are streamed, and all that depends on its rows (their words, resolutions and, for a row
+// it owns, the pose) is loaded before the first store, so a contact waits for two round trips.
 template <bool kFirst>
-__global__ void k_position_fused(DeviceWorld w, dyn_step_params p, uint32_t k, uint32_t sub) {
+__global__ void __launch_bounds__(256) k_position_fused(DeviceWorld w, dyn_step_params p, uint32_t k, uint32_t sub) {
     const uint32_t count = w.ctl[CTL_CONTACTS];
     const size_t n = w.n_cap;
     const int4* pd_prev = w.pd3 + ((k + 2u) % 3u) * n;
     int4* pd_cur = w.pd3 + (k % 3u) * n;
     int4* pd_next = w.pd3 + ((k + 1u) % 3u) * n;
-    const uint32_t* cnt_prev = w.cnt3 + ((k + 2u) % 3u) * n;
-    uint32_t* cnt_cur = w.cnt3 + (k % 3u) * n;
-    uint32_t* cnt_next = w.cnt3 + ((k + 1u) % 3u) * n;
     const float4* res_prev = ((k + 1u) & 1u) ? w.resolution_alt : w.resolution;
     float4* res_cur = (k & 1u) ? w.resolution_alt : w.resolution;
     GRID_STRIDE(i, count) {
-        const uint4 r = w.cur.rows[i];
+        const PositionTerms t = load_position_terms(w, i);
+        const uint32_t pc = position_points(t), own = position_owned(t);
+        if ((pc | own) == 0u) continue;
+        const uint32_t ra = t.rows.x, rb = t.rows.y;
         float4 res_a, res_b;
         if (kFirst) {
-            res_a = w.resolution[r.x];
-            res_b = w.resolution[r.y];
+            res_a = w.resolution[ra];
+            res_b = w.resolution[rb];
             if (w.tape.res) {
-                const uint32_t own = w.cowner[i];
-                if (own & 1u) tape_position_row(w.tape, sub, 0u, r.x, res_a, false, 0u);
-                if (own & 2u) tape_position_row(w.tape, sub, 0u, r.y, res_b, false, 0u);
+                if (own & 1u) tape_position_row(w.tape, sub, 0u, ra, res_a, false, 0u);
+                if (own & 2u) tape_position_row(w.tape, sub, 0u, rb, res_b, false, 0u);
             }
         } else {
-            const RowCorrection ca = row_correction(pd_prev, cnt_prev, r.x);
-            const RowCorrection cb = row_correction(pd_prev, cnt_prev, r.y);
-            res_a = corrected(res_prev[r.x], ca);
-            res_b = corrected(res_prev[r.y], cb);
-            const uint32_t own = w.cowner[i];
-            if (w.tape.res) {
-                if (own & 1u) tape_position_row(w.tape, sub, k, r.x, res_a, true, ca.contributing);
-                if (own & 2u) tape_position_row(w.tape, sub, k, r.y, res_b, true, cb.contributing);
-            }
+            const int4 da = pd_prev[ra], db = pd_prev[rb];
+            res_a = res_prev[ra];
+            res_b = res_prev[rb];
+            float4 pos_a, rot_a, pos_b, rot_b;
             if (own & 1u) {
-                res_cur[r.x] = res_a;
-                move_row(w, r.x, ca);
-                pd_next[r.x] = make_int4(0, 0, 0, 0);
-                cnt_next[r.x] = 0u;
+                pos_a = w.hot[ra].pos;
+                rot_a = w.hot[ra].rot;
             }
             if (own & 2u) {
-                res_cur[r.y] = res_b;
-                move_row(w, r.y, cb);
-                pd_next[r.y] = make_int4(0, 0, 0, 0);
-                cnt_next[r.y] = 0u;
+                pos_b = w.hot[rb].pos;
+                rot_b = w.hot[rb].rot;
+            }
+            const RowCorrection ca = row_correction(da), cb = row_correction(db);
+            res_a = corrected(res_a, ca);
+            res_b = corrected(res_b, cb);
+            if (w.tape.res) {
+                if (own & 1u) tape_position_row(w.tape, sub, k, ra, res_a, true, ca.contributing);
+                if (own & 2u) tape_position_row(w.tape, sub, k, rb, res_b, true, cb.contributing);
+            }
+            if (own & 1u) {
+                res_cur[ra] = res_a;
+                move_row(w, ra, ca, pos_a, rot_a);
+                pd_next[ra] = make_int4(0, 0, 0, 0);
+            }
+            if (own & 2u) {
+                res_cur[rb] = res_b;
+                move_row(w, rb, cb, pos_b, rot_b);
+                pd_next[rb] = make_int4(0, 0, 0, 0);
             }
         }
-        position_block_rows(w, p, i, r, res_a, res_b, pd_cur, cnt_cur);
+        f3 la, lb;
+        if (pc == 0u || !position_correction(p, t, res_a, res_b, &la, &lb)) continue;
+        contribute(pd_cur, ra, __uint_as_float(t.rows.z), la);
+        contribute(pd_cur, rb, __uint_as_float(t.rows.w), lb);
     }
 }
 // The last iteration's correction of every solver row, into the resolution every later pass reads;
@@ -2222,23 +2278,20 @@ __global__ void k_papply_last(DeviceWorld w, uint32_t iterations, uint32_t sub) 
     const size_t n = w.n_cap;
     const uint32_t last = iterations - 1u;
     const int4* pd_last = w.pd3 + (last % 3u) * n;
-    const uint32_t* cnt_last = w.cnt3 + (last % 3u) * n;
     const float4* res_last = (last & 1u) ? w.resolution_alt : w.resolution;
     GRID_STRIDE(i, rows) {
         const uint32_t row = w.solver_rows[i];
-        const RowCorrection c = row_correction(pd_last, cnt_last, row);
+        const int4 words = pd_last[row];
+        const float4 before = res_last[row], at = w.hot[row].pos, turned = w.hot[row].rot;
+        const RowCorrection c = row_correction(words);
         if (w.tape.cnt) {  // a taped step: the last iteration's contributions
             const size_t slot = *w.tape.slot;
             w.tape.cnt[(slot * w.tape.substeps * w.tape.piterations + (size_t)sub * w.tape.piterations + last) * w.tape.n + row] =
                 c.contributing;
         }
-        const float4 res = corrected(res_last[row], c);
-        w.resolution[row] = res;
-        move_row(w, row, c);
-        for (uint32_t b = 0; b < 3u; ++b) {
-            w.pd3[b * n + row] = make_int4(0, 0, 0, 0);
-            w.cnt3[b * n + row] = 0u;
-        }
+        w.resolution[row] = corrected(before, c);
+        move_row(w, row, c, at, turned);
+        for (uint32_t b = 0; b < 3u; ++b) w.pd3[b * n + row] = make_int4(0, 0, 0, 0);
     }
 }
 

@@ -352,6 +352,9 @@ dyn_status ensure_device(dyn_world* w) {
         A(dw.srows.masses, 4 * (size_t)C);
         A(dw.srows.tangent1, C);
         A(dw.srows.tangent2, C);
+        A(dw.srows.pnormal, C);
+        A(dw.srows.prows, C);
+        A(dw.srows.pdepth, C);
         A(dw.parents, N);
         A(dw.istate, N);
         A(dw.live, N);
@@ -363,7 +366,6 @@ dyn_status ensure_device(dyn_world* w) {
         A(dw.contributions, N);
         A(dw.resolution, N);
         A(dw.pd3, 3 * (size_t)N);
-        A(dw.cnt3, 3 * (size_t)N);
         A(dw.resolution_alt, N);
         A(dw.cowner, C);
         // the frozen-contact stores: as many as the contact stream held when the world was made
@@ -846,7 +848,7 @@ void record_step(dyn_world* w, cudaStream_t s, uint32_t parity, bool timed, cons
         if (tape) k_tape_hot<<<blocks_for(d, N, 256), 256, 0, s>>>(dw, *tape, sub);
         k_integrate<<<blocks_for(d, N, 256), 256, 0, s>>>(dw, p);
         const uint32_t st = d->launch.solve_threads;
-        k_solve_prepare<<<blocks_for(d, C, st), st, 0, s>>>(dw);
+        k_solve_prepare<<<blocks_for(d, C, st), st, 0, s>>>(dw, sub == 0u);
         if (sub == 0) {
             mark(ST_WARM);
             if (joint_blocks) k_joints<JP_WARM><<<joint_blocks, 32, 0, s>>>(dw, p);
@@ -1382,7 +1384,8 @@ dyn_status widen_contact_stream(dyn_world* w) {
     }
     ok = ok && grab(&fresh_rows.arm_a, 4 * C * sizeof(float4)) && grab(&fresh_rows.arm_b, 4 * C * sizeof(float4)) &&
          grab(&fresh_rows.masses, 4 * C * sizeof(float4)) && grab(&fresh_rows.tangent1, C * sizeof(float4)) &&
-         grab(&fresh_rows.tangent2, C * sizeof(float4)) && grab(&matched, C * sizeof(uint32_t)) &&
+         grab(&fresh_rows.tangent2, C * sizeof(float4)) && grab(&fresh_rows.pnormal, C * sizeof(float4)) &&
+         grab(&fresh_rows.prows, C * sizeof(uint4)) && grab(&fresh_rows.pdepth, C * sizeof(float4)) && grab(&matched, C * sizeof(uint32_t)) &&
          grab(&cowner, C * sizeof(uint32_t));
     if (!ok) {
         for (void* q : made) cudaFree(q);
@@ -1413,7 +1416,8 @@ dyn_status widen_contact_stream(dyn_world* w) {
     std::vector<void*> stale = {dw.cur.normal, dw.cur.rows, dw.cur.mat, dw.cur.ids, dw.cur.ids2, dw.cur.extra, dw.cur.la,
                                 dw.cur.lb, dw.cur.acc, dw.cur.pos, dw.arc.normal, dw.arc.rows, dw.arc.mat, dw.arc.ids,
                                 dw.arc.ids2, dw.arc.extra, dw.arc.la, dw.arc.lb, dw.arc.acc, dw.arc.pos, dw.srows.arm_a,
-                                dw.srows.arm_b, dw.srows.masses, dw.srows.tangent1, dw.srows.tangent2, dw.matched, dw.cowner};
+                                dw.srows.arm_b, dw.srows.masses, dw.srows.tangent1, dw.srows.tangent2, dw.srows.pnormal, dw.srows.prows,
+                                dw.srows.pdepth, dw.matched, dw.cowner};
     for (void* q : stale) {
         auto it = std::find(d->allocs.begin(), d->allocs.end(), q);
         if (it != d->allocs.end()) d->allocs.erase(it);
