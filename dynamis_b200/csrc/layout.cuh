@@ -75,6 +75,8 @@ enum Ctl : uint32_t {
     CTL_CCD_HITS = 21,       // sweep hits the continuous-collision pass recorded
     CTL_RESTING = 22,        // frozen contacts in the store the next step reads (kept across steps)
     CTL_REST_NEXT = 23,      // frozen contacts this step's commit wrote
+    CTL_CCD_SWEEPS = 24,     // directions of pairs the continuous-collision pass sweeps
+    CTL_CCD_NEXT = 25,       // the next of them
     CTL_COUNT = 32
 };
 

@@ -560,7 +560,7 @@ __device__ Mani box_box_sat(const DBody& fb, const DColl& fc, const DBody& sb, c
 }
 
 // ---- convex support maps (convex.wgsl:1-91) ----
-__device__ f3 support_local(const DeviceWorld& w, const WShape& s, f3 d) {
+__device__ __forceinline__ f3 support_primitive(const WShape& s, f3 d) {
     if (s.kind == 1u) return normalize(d) * s.radius;
     if (s.kind == 2u) {
         f3 signs = mk3(d.x > 0.0f ? 1.0f : -1.0f, d.y > 0.0f ? 1.0f : -1.0f, d.z > 0.0f ? 1.0f : -1.0f);
@@ -570,12 +570,13 @@ __device__ f3 support_local(const DeviceWorld& w, const WShape& s, f3 d) {
         f3 tip = mk3(0.0f, 1.0f, 0.0f) * s.half_height * (d.y > 0.0f ? 1.0f : -1.0f);
         return tip + normalize(d) * s.radius;
     }
-    if (s.kind == 4u) {
-        f3 base = mk3(0.0f, 1.0f, 0.0f) * s.half_height * (d.y > 0.0f ? 1.0f : -1.0f);
-        f3 radial = d - mk3(0.0f, d.y, 0.0f);
-        if (length(radial) < 1e-6f) return base;
-        return base + normalize(radial) * s.radius;
-    }
+    f3 base = mk3(0.0f, 1.0f, 0.0f) * s.half_height * (d.y > 0.0f ? 1.0f : -1.0f);
+    f3 radial = d - mk3(0.0f, d.y, 0.0f);
+    if (length(radial) < 1e-6f) return base;
+    return base + normalize(radial) * s.radius;
+}
+__device__ f3 support_local(const DeviceWorld& w, const WShape& s, f3 d) {
+    if (s.kind <= 4u) return support_primitive(s, d);
     const dyn_shape_source_record& src = w.sources[s.source];
     const float4* verts = w.vertices + src.vertex_offset;
     const uint32_t count = src.vertex_count;
@@ -921,6 +922,25 @@ __device__ EpaOut penetration_probe(const DeviceWorld& w, const WShape& first, c
     return best;
 }
 
+// GJK's fixed points. The reference's search either ends within a dozen iterations or, for about one
+// pair in five that reach it, meets a simplex that an iteration turns into itself: the reduction drops
+// the newest point and the support point that replaces it is that point again. An iteration depends
+// on the points w alone (their closest point gives the direction, the tests compare w and v), so the
+// reference repeats this one until its limit of 24 ends the walk with the simplex unchanged; here the
+// walk ends at once. Tells whether the points `lam` keeps are all but the newest and the support
+// point equals that one bit for bit.
+constexpr uint32_t kGjkIterations = 24u;
+__device__ __forceinline__ bool gjk_repeats(const float* lam, uint32_t count, f3 newest, f3 support_point) {
+    bool repeats = count >= 2u;
+#pragma unroll
+    for (uint32_t i = 0; i < 4u; ++i) {
+        if (i < count) repeats = repeats && ((lam[i] > 1e-6f) == (i + 1u < count));
+    }
+    return repeats && __float_as_uint(newest.x) == __float_as_uint(support_point.x) &&
+           __float_as_uint(newest.y) == __float_as_uint(support_point.y) &&
+           __float_as_uint(newest.z) == __float_as_uint(support_point.z);
+}
+
 // convex.wgsl:464-521 then 584-618
 __device__ Hit convex_hit(const DeviceWorld& w, const WShape& first, const WShape& second) {
     SPt s[4];
@@ -935,7 +955,7 @@ __device__ Hit convex_hit(const DeviceWorld& w, const WShape& first, const WShap
     count = 1;
     SRes cl = simplex_closest(s, count);
     float tiny = 1e-4f * wmin(shape_scale(first), shape_scale(second));
-    for (uint32_t iter = 0; iter < 24u; ++iter) {
+    for (uint32_t iter = 0; iter < kGjkIterations; ++iter) {
         if (cl.pen || length(cl.v) < tiny) {
             while (count < 4u) {
                 f3 d = simplex_expand_dir(s, count);
@@ -956,6 +976,7 @@ __device__ Hit convex_hit(const DeviceWorld& w, const WShape& first, const WShap
             if (rdist > 1e-6f) rnormal = sign_normalize(cl.pb - cl.pa);
             break;
         }
+        const bool repeats = gjk_repeats(cl.lam, count, s[count - 1u].w, sp.w);
         // simplex_reduce
         SPt kept[4];
         uint32_t kc = 0;
@@ -985,6 +1006,7 @@ __device__ Hit convex_hit(const DeviceWorld& w, const WShape& first, const WShap
         }
         s[count] = sp;
         count += 1;
+        if (repeats) break;
         cl = simplex_closest(s, count);
     }
     if (!rpen) {
@@ -1057,7 +1079,7 @@ __device__ GjkOut gjk_phase(const DeviceWorld& w, const WShape& first, const WSh
     }
     SRes cl = simplex_closest(o.s, o.count);
     float tiny = 1e-4f * wmin(shape_scale(first), shape_scale(second));
-    for (uint32_t iter = 0; iter < 24u; ++iter) {
+    for (uint32_t iter = 0; iter < kGjkIterations; ++iter) {
         if (cl.pen || length(cl.v) < tiny) {
             while (o.count < 4u) {
                 f3 d = simplex_expand_dir(o.s, o.count);
@@ -1078,6 +1100,7 @@ __device__ GjkOut gjk_phase(const DeviceWorld& w, const WShape& first, const WSh
             if (o.dist > 1e-6f) o.normal = sign_normalize(cl.pb - cl.pa);
             break;
         }
+        const bool repeats = gjk_repeats(cl.lam, o.count, o.s[o.count - 1u].w, sp.w);
         SPt kept[4];
         uint32_t kc = 0;
         for (uint32_t i = 0; i < 4; ++i) {
@@ -1105,6 +1128,7 @@ __device__ GjkOut gjk_phase(const DeviceWorld& w, const WShape& first, const WSh
         }
         o.s[o.count] = sp;
         o.count += 1;
+        if (repeats) break;
         cl = simplex_closest(o.s, o.count);
     }
     return o;
@@ -1174,30 +1198,249 @@ __device__ __forceinline__ uint32_t warp_first_max(const Lanes<G>& L, uint32_t k
     return L.min(key == top ? index : 0xFFFFFFFFu);
 }
 
-// support_local over a hull with the warp's lanes striding the vertices; the reduction keeps the
-// sequential scan's choice: the largest dot product, the lowest index among equal ones.
+// A shape as a lane group searches it: a hull's vertices lie over the lanes (vertex i on lane
+// i % G), the first 32 of them in registers, loaded once for all of a pair's evaluations.
 template <uint32_t G>
-__device__ __forceinline__ f3 warp_support_local(const Lanes<G>& L, const DeviceWorld& w, const WShape& s, f3 d) {
-    if (s.kind != 5u) return support_local(w, s, d);
-    const dyn_shape_source_record& src = w.sources[s.source];
-    const float4* verts = w.vertices + src.vertex_offset;
+struct GroupShape : WShape {
+    static constexpr uint32_t kHeld = 32u / G;
+    const float4* verts;
+    uint32_t count;  // vertices of a hull, 0 for the other kinds
+    f3 held[kHeld];
+};
+template <uint32_t G>
+__device__ __forceinline__ GroupShape<G> group_shape(const Lanes<G>& L, const DeviceWorld& w, const WShape& s) {
+    GroupShape<G> g;
+    static_cast<WShape&>(g) = s;
+    g.verts = nullptr;
+    g.count = 0u;
+    if (s.kind == 5u) {
+        const dyn_shape_source_record& src = w.sources[s.source];
+        g.verts = w.vertices + src.vertex_offset;
+        g.count = src.vertex_count;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < GroupShape<G>::kHeld; ++k) {
+        const uint32_t i = L.lane + k * G;
+        g.held[k] = i < g.count ? xyz(__ldg(g.verts + i)) : s3(0.0f);
+    }
+    return g;
+}
+// A lane's best vertex along d: the largest dot product, the lowest index among equal ones. The
+// group's reduction over these keeps the sequential scan's choice.
+struct LaneBest {
+    uint32_t key, index;
+    f3 v;
+};
+template <uint32_t G>
+__device__ __forceinline__ LaneBest lane_best(const Lanes<G>& L, const GroupShape<G>& s, f3 d) {
     float best = -3.402823466e38f;
-    uint32_t bi = 0xFFFFFFFFu;
-    for (uint32_t i = L.lane; i < src.vertex_count; i += G) {
-        float sd = dot(xyz(__ldg(verts + i)), d);
-        if (sd > best) {
+    LaneBest r{0u, 0xFFFFFFFFu, s3(0.0f)};
+#pragma unroll
+    for (uint32_t k = 0; k < GroupShape<G>::kHeld; ++k) {
+        const uint32_t i = L.lane + k * G;
+        const float sd = dot(s.held[k], d);
+        if (i < s.count && sd > best) {
             best = sd;
-            bi = i;
+            r.index = i;
+            r.v = s.held[k];
         }
     }
-    bi = warp_first_max(L, bi == 0xFFFFFFFFu ? 0u : order_key(best), bi);
-    return bi == 0xFFFFFFFFu ? s3(0.0f) : xyz(__ldg(verts + bi));
+    for (uint32_t i = L.lane + 32u; i < s.count; i += G) {
+        const f3 v = xyz(__ldg(s.verts + i));
+        const float sd = dot(v, d);
+        if (sd > best) {
+            best = sd;
+            r.index = i;
+            r.v = v;
+        }
+    }
+    if (r.index != 0xFFFFFFFFu) r.key = order_key(best);
+    return r;
 }
 template <uint32_t G>
-__device__ __forceinline__ f3 warp_support(const Lanes<G>& L, const DeviceWorld& w, const WShape& s, f3 direction) {
-    f3 local_d = quat_rotate(quat_conj(s.rotation), direction);
-    f3 local = warp_support_local(L, w, s, local_d * s.scale);
+__device__ __forceinline__ f3 group_vertex(const Lanes<G>& L, const LaneBest& b, uint32_t top, uint32_t index) {
+    const uint32_t from = index & (G - 1u);
+    const f3 v = mk3(L.shfl(b.v.x, from), L.shfl(b.v.y, from), L.shfl(b.v.z, from));
+    return top == 0u ? s3(0.0f) : v;
+}
+template <uint32_t G>
+__device__ __forceinline__ f3 warp_support(const Lanes<G>& L, const GroupShape<G>& s, f3 direction) {
+    const f3 d = quat_rotate(quat_conj(s.rotation), direction) * s.scale;
+    f3 local;
+    if (s.kind == 5u) {
+        const LaneBest b = lane_best(L, s, d);
+        const uint32_t top = L.max(b.key);
+        local = group_vertex(L, b, top, L.min(b.key == top ? b.index : 0xFFFFFFFFu));
+    } else {
+        local = support_primitive(s, d);
+    }
     return s.center + quat_rotate(s.rotation, local * s.scale);
+}
+// Both supports of a pair, their independent reductions interleaved.
+template <uint32_t G>
+__device__ __forceinline__ void group_supports(const Lanes<G>& L, const GroupShape<G>& first, const GroupShape<G>& second, f3 direction,
+                                               f3* a, f3* b) {
+    const f3 da = quat_rotate(quat_conj(first.rotation), direction) * first.scale;
+    const f3 db = quat_rotate(quat_conj(second.rotation), -direction) * second.scale;
+    f3 la, lb;
+    if ((first.count | second.count) != 0u) {
+        const LaneBest ba = lane_best(L, first, da), bb = lane_best(L, second, db);
+        const uint32_t ta = L.max(ba.key), tb = L.max(bb.key);
+        const uint32_t ia = L.min(ba.key == ta ? ba.index : 0xFFFFFFFFu), ib = L.min(bb.key == tb ? bb.index : 0xFFFFFFFFu);
+        la = group_vertex(L, ba, ta, ia);
+        lb = group_vertex(L, bb, tb, ib);
+    }
+    if (first.kind != 5u) la = support_primitive(first, da);
+    if (second.kind != 5u) lb = support_primitive(second, db);
+    *a = first.center + quat_rotate(first.rotation, la * first.scale);
+    *b = second.center + quat_rotate(second.rotation, lb * second.scale);
+}
+
+// ---- GJK on a lane group ----
+// The closest point of a simplex is the first shortest of up to fourteen candidates: four vertices,
+// six edges, four triangles, in that order (simplex_closest). A lane group evaluates them side by
+// side, one lane per candidate, with the arithmetic of the sequential scan, and keeps the shortest
+// with the lowest candidate number, which is the candidate the scan's strict comparison keeps. The
+// simplex lies in shared memory (dynamically indexed points would spill from registers).
+// candidate: its points, and their count in the last entry
+__constant__ uint8_t kCandidate[14][4] = {{0, 0, 0, 1}, {1, 1, 1, 1}, {2, 2, 2, 1}, {3, 3, 3, 1}, {0, 1, 1, 2}, {0, 2, 2, 2}, {0, 3, 3, 2},
+                                          {1, 2, 2, 2}, {1, 3, 3, 2}, {2, 3, 3, 2}, {0, 1, 2, 3}, {0, 1, 3, 3}, {0, 2, 3, 3}, {1, 2, 3, 3}};
+__constant__ uint8_t kTetraFace[4][3] = {{0, 1, 2}, {0, 2, 3}, {0, 3, 1}, {1, 3, 2}};
+
+struct GroupClosest {  // SRes, the same on every lane of the group, except `ab`
+    f3 v;
+    float len;  // length(v)
+    float lam[4];
+    bool pen;
+    float ab;  // lanes 0-2: pa's components, lanes 3-5: pb's
+};
+// A lane's candidates, fixed for a kernel: lane, lane + G, ... in kCandidate, packed a byte a point.
+template <uint32_t G>
+struct LaneCandidates {
+    static constexpr uint32_t kRounds = (14u + G - 1u) / G;
+    uint32_t packed[kRounds];  // 0xFFFFFFFF: none
+    __device__ __forceinline__ explicit LaneCandidates(const Lanes<G>& L) {
+#pragma unroll
+        for (uint32_t r = 0; r < kRounds; ++r) {
+            const uint32_t c = r * G + L.lane;
+            packed[r] = c < 14u ? (uint32_t)kCandidate[c][0] | (uint32_t)kCandidate[c][1] << 8 | (uint32_t)kCandidate[c][2] << 16 |
+                                      (uint32_t)kCandidate[c][3] << 24
+                                : 0xFFFFFFFFu;
+        }
+    }
+};
+template <uint32_t G>
+__device__ __forceinline__ GroupClosest group_closest(const Lanes<G>& L, const LaneCandidates<G>& mine, const SPt* s, uint32_t count) {
+    GroupClosest r;
+    r.pen = false;
+    if (count == 4u) {  // tetra_contains, a face per lane
+        bool out = false;
+        if (L.lane < 4u) {
+            const f3 a = s[kTetraFace[L.lane][0]].w, b = s[kTetraFace[L.lane][1]].w, c = s[kTetraFace[L.lane][2]].w;
+            const f3 normal = cross(b - a, c - a);
+            const float span = face_span(a, b, c);
+            out = length(normal) <= 1e-6f * span * span || dot(normal, s3(0.0f) - a) > 0.0f;
+        }
+        r.pen = !L.any(out);
+    }
+    if (r.pen) {
+        r.v = s3(0.0f);
+        r.len = 0.0f;
+        for (int i = 0; i < 4; ++i) r.lam[i] = 0.0f;
+        r.ab = 0.0f;
+        return r;
+    }
+    f3 v = s3(3.402823466e38f);
+    float len = __int_as_float(0x7F800000);
+    f3 wts = s3(0.0f);
+    uint32_t best = 0xFFFFFFFFu, best_points = 0u;
+#pragma unroll
+    for (uint32_t round = 0; round < LaneCandidates<G>::kRounds; ++round) {
+        const uint32_t packed = mine.packed[round];
+        const uint32_t i = packed & 255u, j = (packed >> 8) & 255u, k = (packed >> 16) & 255u, points = packed >> 24;
+        if (k >= count) continue;
+        const f3 a = s[i].w;
+        f3 point = a, wt = mk3(1.0f, 0.0f, 0.0f);
+        if (points == 2u) {
+            const f3 ab = s[j].w - a;
+            const float denom = dot(ab, ab);
+            if (denom < 1e-12f) continue;
+            const float t = wclamp(-dot(a, ab) / denom, 0.0f, 1.0f);
+            point = a + ab * t;
+            wt = mk3(1.0f - t, t, 0.0f);
+        } else if (points == 3u) {
+            point = closest_on_triangle(a, s[j].w, s[k].w, &wt);
+        }
+        const float l = length(point);
+        if (l < len) {
+            len = l;
+            v = point;
+            wts = wt;
+            best = round * G + L.lane;
+            best_points = packed;
+        }
+    }
+    // lengths are non-negative, so their bits order as they do; no candidate keeps the scan's start
+    const uint32_t key = best == 0xFFFFFFFFu ? 0xFFFFFFFFu : __float_as_uint(len);
+    const uint32_t least = L.min(key);
+    const uint32_t winner = L.min(key == least ? best : 0xFFFFFFFFu);
+    const uint32_t from = winner & (G - 1u);  // candidate c lives on lane c % G
+    r.v = mk3(L.shfl(v.x, from), L.shfl(v.y, from), L.shfl(v.z, from));
+    const float x = L.shfl(wts.x, from), y = L.shfl(wts.y, from), z = L.shfl(wts.z, from);
+    const uint32_t chosen = L.shfl(best_points, from);
+    if (winner == 0xFFFFFFFFu) {
+        r.v = s3(3.402823466e38f);
+        r.len = __int_as_float(0x7F800000);
+        for (int i = 0; i < 4; ++i) r.lam[i] = 0.0f;
+    } else {
+        r.len = __uint_as_float(least);
+        const uint32_t i = chosen & 255u, j = (chosen >> 8) & 255u, k = (chosen >> 16) & 255u, points = chosen >> 24;
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; ++q) r.lam[q] = q == i ? x : (points > 1u && q == j ? y : (points > 2u && q == k ? z : 0.0f));
+    }
+    // pa and pb, a component per lane, in point order
+    r.ab = 0.0f;
+    if (L.lane < 6u) {
+#pragma unroll
+        for (uint32_t q = 0; q < 4u; ++q) {
+            if (q < count) r.ab = r.ab + r.lam[q] * (L.lane < 3u ? comp(s[q].a, L.lane) : comp(s[q].b, L.lane - 3u));
+        }
+    }
+    return r;
+}
+template <uint32_t G>
+__device__ __forceinline__ SPt group_support_pair(const Lanes<G>& L, const GroupShape<G>& first, const GroupShape<G>& second, f3 d) {
+    f3 a, b;
+    group_supports(L, first, second, d, &a, &b);
+    return SPt{a - b, a, b};
+}
+// simplex_reduce: the points with weight, in order; the first point when none has any. Returns their count.
+template <uint32_t G>
+__device__ __forceinline__ uint32_t group_reduce(const Lanes<G>& L, SPt* s, const float* lam) {
+    const uint32_t keep = (lam[0] > 1e-6f ? 1u : 0u) | (lam[1] > 1e-6f ? 2u : 0u) | (lam[2] > 1e-6f ? 4u : 0u) | (lam[3] > 1e-6f ? 8u : 0u);
+    const bool mine = L.lane < 4u && ((keep >> L.lane) & 1u);
+    SPt p;
+    if (mine) p = s[L.lane];
+    L.sync();
+    if (mine) s[__popc(keep & ((1u << L.lane) - 1u))] = p;
+    L.sync();
+    return keep ? __popc(keep) : 1u;
+}
+// simplex_holds: does the simplex already hold this support point?
+template <uint32_t G>
+__device__ __forceinline__ bool group_holds(const Lanes<G>& L, const SPt* s, uint32_t count, f3 point, float span) {
+    const float tol = (1e-5f * span) * (1e-5f * span);
+    bool holds = false;
+    if (L.lane < count) {
+        const f3 off = s[L.lane].w - point;
+        holds = dot(off, off) <= tol;
+    }
+    return L.any(holds);
+}
+template <uint32_t G>
+__device__ __forceinline__ void group_push(const Lanes<G>& L, SPt* s, uint32_t at, const SPt& p) {
+    if (L.lane == 0u) s[at] = p;
+    L.sync();
 }
 
 struct EpaWarpShared {
@@ -1251,8 +1494,8 @@ __device__ __forceinline__ void warp_best_face(const Lanes<G>& L, const EpaWarpS
 
 // convex.wgsl:286-437 on one warp. All lanes return the same result.
 template <uint32_t G>
-__device__ EpaOut warp_epa(const Lanes<G>& L, const DeviceWorld& w, const WShape& first, const WShape& second,
-                           const f3* simplex, EpaWarpShared& m) {
+__device__ EpaOut warp_epa(const Lanes<G>& L, const GroupShape<G>& first, const GroupShape<G>& second, const f3* simplex,
+                           EpaWarpShared& m) {
     const uint32_t lane = L.lane;
     const uint32_t lt = (1u << lane) - 1u;
     EpaOut invalid{false, mk3(0.0f, 1.0f, 0.0f), 0.0f};
@@ -1281,7 +1524,7 @@ __device__ EpaOut warp_epa(const Lanes<G>& L, const DeviceWorld& w, const WShape
     for (uint32_t iter = 0; iter < 32u; ++iter) {
         warp_best_face(L, m, fcount, &bd, &bf);
         f3 n = xyz(m.fn[bf]);
-        f3 probe = warp_support(L, w, first, n) - warp_support(L, w, second, -n);
+        const f3 probe = group_support_pair(L, first, second, n).w;
         float gain = dot(probe, n) - bd;
         if (gain < 1e-4f) break;
         if (vc >= 64u) break;
@@ -1379,25 +1622,24 @@ __device__ EpaOut warp_epa(const Lanes<G>& L, const DeviceWorld& w, const WShape
 }
 
 template <uint32_t G>
-__device__ __forceinline__ float warp_projection_depth(const Lanes<G>& L, const DeviceWorld& w, const WShape& f, const WShape& s,
-                                                       f3 direction) {
+__device__ __forceinline__ float warp_projection_depth(const Lanes<G>& L, const GroupShape<G>& f, const GroupShape<G>& s, f3 direction) {
     f3 n = normalize(direction);
-    return dot(warp_support(L, w, f, n) - warp_support(L, w, s, -n), n);
+    return dot(group_support_pair(L, f, s, n).w, n);
 }
 
 // convex.wgsl:602-617 after a penetrating GJK (one warp, every lane returns the same hit).
 template <uint32_t G>
-__device__ Hit warp_penetrating_hit(const Lanes<G>& L, const DeviceWorld& w, const WShape& first, const WShape& second,
+__device__ Hit warp_penetrating_hit(const Lanes<G>& L, const DeviceWorld& w, const GroupShape<G>& first, const GroupShape<G>& second,
                                     const f3* simplex, EpaWarpShared& m) {
-    EpaOut epa = warp_epa(L, w, first, second, simplex, m);
+    EpaOut epa = warp_epa(L, first, second, simplex, m);
     Hit result;
     bool accept = epa.valid && epa.depth > 0.0f && epa.depth < 3.402823466e38f && length(epa.normal) > 0.5f;
     if (accept) {
-        accept = epa.depth < warp_projection_depth(L, w, first, second, epa.normal) + 0.1f * wmin(shape_scale(first), shape_scale(second));
+        accept = epa.depth < warp_projection_depth(L, first, second, epa.normal) + 0.1f * wmin(shape_scale(first), shape_scale(second));
     }
     if (accept) {
-        f3 pa = warp_support(L, w, first, epa.normal);
-        f3 pb = warp_support(L, w, second, -epa.normal);
+        f3 pa, pb;
+        group_supports(L, first, second, epa.normal, &pa, &pb);
         result = Hit{-epa.depth, (pa + pb) * 0.5f, epa.normal};
     } else {
         // convex_penetration_probe over the four-point simplex, centre direction and six axes: each
@@ -1428,12 +1670,105 @@ __device__ Hit warp_penetrating_hit(const Lanes<G>& L, const DeviceWorld& w, con
             }
         }
         const f3 best_normal = best_i < pc ? normalize(probed[best_i]) : mk3(0.0f, 1.0f, 0.0f);
-        f3 pa = warp_support(L, w, first, best_normal);
-        f3 pb = warp_support(L, w, second, -best_normal);
+        f3 pa, pb;
+        group_supports(L, first, second, best_normal, &pa, &pb);
         result = Hit{-best_depth, (pa + pb) * 0.5f, best_normal};
     }
     if (dot(result.normal, second.center - first.center) < 0.0f) result.normal = -result.normal;
     return result;
+}
+
+// convex_hit (convex.wgsl:464-521, 584-618) on a lane group: the same hit on every lane. `s` is the
+// group's simplex in shared memory.
+template <uint32_t G>
+__device__ Hit group_convex_hit(const Lanes<G>& L, const DeviceWorld& w, const GroupShape<G>& first, const GroupShape<G>& second,
+                                SPt* s, EpaWarpShared& m) {
+    const LaneCandidates<G> mine(L);
+    f3 dir = second.center - first.center;
+    f3 normal = sign_normalize(dir);
+    if (length(dir) < 1e-8f) dir = mk3(1.0f, 0.0f, 0.0f);
+    f3 pa = first.center, pb = second.center;
+    float dist = 0.0f;
+    bool pen = false;
+    SPt sp = group_support_pair(L, first, second, dir);
+    L.sync();
+    group_push(L, s, 0u, sp);
+    uint32_t count = 1u;
+    GroupClosest cl = group_closest(L, mine, s, count);
+    const float tiny = 1e-4f * wmin(shape_scale(first), shape_scale(second));
+    for (uint32_t iter = 0; iter < kGjkIterations; ++iter) {
+        if (cl.pen || cl.len < tiny) {
+            while (count < 4u) {
+                sp = group_support_pair(L, first, second, simplex_expand_dir(s, count));
+                L.sync();
+                group_push(L, s, count, sp);
+                count += 1u;
+            }
+            pen = true;
+            break;
+        }
+        sp = group_support_pair(L, first, second, -cl.v);
+        bool done = dot(sp.w, -cl.v) <= dot(cl.v, -cl.v) + 1e-4f * wmax(1.0f, dot(cl.v, cl.v));
+        const bool repeats = gjk_repeats(cl.lam, count, s[count - 1u].w, sp.w);
+        if (!done) {
+            count = group_reduce(L, s, cl.lam);
+            done = group_holds(L, s, count, sp.w, shape_scale(second));
+        }
+        if (done) {
+            dist = cl.len;
+            pa = mk3(L.shfl(cl.ab, 0u), L.shfl(cl.ab, 1u), L.shfl(cl.ab, 2u));
+            pb = mk3(L.shfl(cl.ab, 3u), L.shfl(cl.ab, 4u), L.shfl(cl.ab, 5u));
+            if (dist > 1e-6f) normal = sign_normalize(pb - pa);
+            break;
+        }
+        group_push(L, s, count, sp);
+        count += 1u;
+        if (repeats) break;
+        cl = group_closest(L, mine, s, count);
+    }
+    if (pen) {
+        const f3 simplex[4] = {s[0].w, s[1].w, s[2].w, s[3].w};
+        L.sync();
+        return warp_penetrating_hit(L, w, first, second, simplex, m);
+    }
+    // penetration_probe (convex.wgsl:532-582), a direction per lane: simplex triples, the centre axis,
+    // the six axes. Any direction without overlap makes the minimum non-positive, which is all the
+    // caller asks; otherwise the first minimum in direction order.
+    f3 d = s3(0.0f);
+    bool probes = false;
+    if (L.lane < 4u) {
+        const uint32_t i = kCandidate[10u + L.lane][0], j = kCandidate[10u + L.lane][1], k = kCandidate[10u + L.lane][2];
+        if (k < count) {
+            d = cross(s[j].w - s[i].w, s[k].w - s[i].w);
+            probes = length(d) > 1e-8f;
+        }
+    } else if (L.lane == 4u) {
+        d = second.center - first.center;
+        probes = length(d) > 1e-8f;
+    } else if (L.lane < 11u) {
+        const uint32_t x = L.lane - 5u;
+        const float sign = (x & 1u) ? -1.0f : 1.0f;
+        d = mk3((x >> 1) == 0u ? sign : 0.0f, (x >> 1) == 1u ? sign : 0.0f, (x >> 1) == 2u ? sign : 0.0f);
+        probes = true;
+    }
+    const float depth = probes ? support_projection_depth(w, first, second, d) : 3.402823466e38f;
+    if (!L.any(probes && depth <= 0.0f)) {
+        // positive depths only (or NaN, which the scan's comparison never keeps)
+        const uint32_t key = probes && depth < 3.402823466e38f ? __float_as_uint(depth) : 0xFFFFFFFFu;
+        const uint32_t least = L.min(key);
+        float best = 3.402823466e38f;
+        f3 axis = mk3(0.0f, 1.0f, 0.0f);
+        if (least != 0xFFFFFFFFu) {
+            best = __uint_as_float(least);
+            const uint32_t from = L.min(key == least ? L.lane : 0xFFFFFFFFu);
+            const f3 n = probes ? normalize(d) : s3(0.0f);
+            axis = mk3(L.shfl(n.x, from), L.shfl(n.y, from), L.shfl(n.z, from));
+        }
+        if (dot(axis, second.center - first.center) < 0.0f) axis = -axis;
+        return Hit{-best, (pa + pb) * 0.5f, axis};
+    }
+    if (dist > 0.0f) return Hit{dist, (pa + pb) * 0.5f, normal};
+    return Hit{3.402823466e38f, s3(0.0f), s3(0.0f)};
 }
 
 // ---- features (convex.wgsl:639-900) ----

@@ -944,22 +944,93 @@ __device__ __forceinline__ void push_hit(const DeviceWorld& w, uint32_t index, c
 // the rounding of support points at world coordinates of a few hundred metres (~1e-5 m).
 constexpr float kRejectTolerance = 1e-3f;
 
-// Phase 1: GJK per pair (convex.wgsl:464-521) and, for separated shapes, the penetration probe
-// (convex.wgsl:532-582, 588-600); penetrating pairs queue for EPA.
+// Phase 1: GJK per pair (convex.wgsl:464-521); separated pairs queue for the penetration probe
+// (convex.wgsl:532-582, 588-600), penetrating ones for EPA.
 //
 // The work of one pair is a sequence of support-pair evaluations: the first along the centre axis,
-// one per GJK iteration along -v, up to three that grow a penetrating simplex to a tetrahedron, and
-// one per probe direction. Each lane runs its pair as a state machine that makes exactly one
-// support-pair evaluation per trip of the loop below, and a lane whose pair is done takes the next
-// pair from the convex list through a shared ticket. So the lanes of a warp keep evaluating
-// supports together instead of waiting for the warp's slowest pair, whatever their pairs' iteration
-// counts. Each state does the same arithmetic, in the same order, as gjk_phase followed by
-// separated_hit (narrow.cuh); only the interleaving of pairs on a lane changes.
+// one per GJK iteration along -v, and up to three that grow a penetrating simplex to a tetrahedron.
+// A group of kGjkLanes lanes runs one pair as a state machine that makes one evaluation per trip of
+// the loop below, so the groups of a warp meet at the evaluation whatever their pairs' states, and
+// a group whose pair is done takes the next one through a shared ticket. Within an evaluation the
+// lanes stride the hulls' vertices, and a simplex's fourteen closest-point candidates go one to a
+// lane (group_closest). A trip is bound by the latency of dependent arithmetic (correctly rounded
+// divisions and roots) and of the vertex loads: on one lane it took about 8 us, so that the slowest
+// pair of even a 64-body heap held the step for 190 us.
 enum GjkState : uint32_t { GS_IDLE = 0, GS_FIRST = 1, GS_ITER = 2, GS_EXPAND = 3 };
-// simplex triples in the probe's order (i < j < k ascending), one per bit of GjkLane::triples
+// simplex triples in the probe's order (i < j < k ascending), one per bit of the probe's triples
 __constant__ uint8_t kProbeTriple[4][3] = {{0, 1, 2}, {0, 1, 3}, {0, 2, 3}, {1, 2, 3}};
 constexpr uint32_t kProbeCentre = 4u, kProbeAxes = 5u, kProbeEnd = 11u;
 
+constexpr uint32_t kGjkThreads = 128;
+// Below this many pairs a group each is faster, above it a lane each: 2,849 pairs (the 4,913-body pile)
+// 49 against 143 us, 23,599 (32,768 bodies) 223 against 187 us, 107,873 (262,144 bodies) 973 against
+// 253 us; 4 blocks of 8 groups per SM are 4,736 pairs at a time.
+constexpr uint32_t kGjkGroupPairs = 8192;
+constexpr uint32_t kGjkLanes = 16;
+constexpr uint32_t kGjkGroups = kGjkThreads / kGjkLanes;
+
+struct GjkGroup {
+    uint32_t state, index, count, iter;
+    float tiny, margin;
+    GroupClosest cl;
+    GroupShape<kGjkLanes> a, b;
+    SPt* s;  // the simplex (4 points), the group's slice of shared memory
+};
+
+// A pair that GJK leaves separated, or that runs out of iterations, goes to the penetration probe's
+// queue with its simplex, its closest points and its normal (k_convex_probe).
+__device__ __forceinline__ void gjk_to_probe(const Lanes<kGjkLanes>& L, const DeviceWorld& w, GjkGroup& g, float dist, f3 pa, f3 pb,
+                                             f3 normal) {
+    uint32_t slot = 0u;
+    if (L.lane == 0u) slot = atomicAdd(&w.ctl[CTL_PROBES], 1u);
+    slot = L.shfl(slot, 0u);
+    if (L.lane == 0u) w.probe_list[slot] = g.index;
+    float4* q = w.probe_data + 6 * (size_t)slot;
+    if (L.lane < 4u) {
+        const float word = L.lane == 0u ? __uint_as_float(g.count) : (L.lane == 1u ? dist : (L.lane == 2u ? pa.x : pa.y));
+        q[L.lane] = mk4(L.lane < g.count ? g.s[L.lane].w : s3(0.0f), word);
+    } else if (L.lane == 4u) {
+        q[4] = mk4(pb, pa.z);
+    } else if (L.lane == 5u) {
+        q[5] = mk4(normal, 0.0f);
+    }
+    g.state = GS_IDLE;
+}
+// A penetrating pair with its tetrahedron complete goes to the EPA queue.
+__device__ __forceinline__ void gjk_to_epa(const Lanes<kGjkLanes>& L, const DeviceWorld& w, GjkGroup& g) {
+    uint32_t slot = 0u;
+    if (L.lane == 0u) slot = atomicAdd(&w.ctl[CTL_EPA], 1u);
+    slot = L.shfl(slot, 0u);
+    if (L.lane == 0u) w.epa_list[slot] = g.index;
+    if (L.lane < 4u) w.epa_simplex[4 * (size_t)slot + L.lane] = mk4(g.s[L.lane].w, 0.0f);
+    g.state = GS_IDLE;
+}
+// The loop head of gjk_phase: terminate, grow a penetrating simplex, or take another iteration.
+__device__ __forceinline__ void gjk_head(const Lanes<kGjkLanes>& L, const DeviceWorld& w, GjkGroup& g) {
+    if (g.iter >= kGjkIterations) {
+        gjk_to_probe(L, w, g, 0.0f, g.a.center, g.b.center, sign_normalize(g.b.center - g.a.center));
+    } else if (g.cl.pen || g.cl.len < g.tiny) {
+        if (g.count < 4u) {
+            g.state = GS_EXPAND;
+        } else {
+            gjk_to_epa(L, w, g);
+        }
+    } else {
+        g.state = GS_ITER;
+    }
+}
+__device__ __forceinline__ void gjk_separated(const Lanes<kGjkLanes>& L, const DeviceWorld& w, GjkGroup& g) {
+    const f3 pa = mk3(L.shfl(g.cl.ab, 0u), L.shfl(g.cl.ab, 1u), L.shfl(g.cl.ab, 2u));
+    const f3 pb = mk3(L.shfl(g.cl.ab, 3u), L.shfl(g.cl.ab, 4u), L.shfl(g.cl.ab, 5u));
+    f3 normal = sign_normalize(g.b.center - g.a.center);
+    if (g.cl.len > 1e-6f) normal = sign_normalize(pb - pa);
+    gjk_to_probe(L, w, g, g.cl.len, pa, pb, normal);
+}
+
+// The same machine with one lane per pair, for batches that fill the chip: fewer instructions per
+// pair than a group spends (every lane of a group repeats the rotations and the tests), but a trip
+// takes the union of a warp's states and candidates. Each state does the same arithmetic, in the same
+// order, as gjk_phase followed by separated_hit (narrow.cuh).
 struct GjkLane {
     uint32_t state, index, count, iter;
     float tiny, margin, dist;
@@ -971,7 +1042,6 @@ struct GjkLane {
 // Each lane's simplex lives in shared memory at an odd word stride (37 words for 36 used), so the
 // lanes of a warp reading the same point land in different banks; held in the lane's registers it
 // would be indexed by the simplex size and spill to local memory.
-constexpr uint32_t kGjkThreads = 128;
 constexpr uint32_t kSimplexStride = 37;
 static_assert(sizeof(SPt) * 4 <= kSimplexStride * sizeof(float), "a lane's simplex fits its slice");
 
@@ -998,7 +1068,7 @@ __device__ __forceinline__ void gjk_to_epa(const DeviceWorld& w, GjkLane& L) {
 }
 // The loop head of gjk_phase: terminate, grow a penetrating simplex, or take another iteration.
 __device__ __forceinline__ void gjk_head(const DeviceWorld& w, GjkLane& L) {
-    if (L.iter >= 24u) {
+    if (L.iter >= kGjkIterations) {
         gjk_to_probe(w, L);
     } else if (L.cl.pen || length(L.cl.v) < L.tiny) {
         if (L.count < 4u) {
@@ -1040,9 +1110,86 @@ __global__ void __launch_bounds__(128) k_convex_reject(DeviceWorld w, dyn_step_p
     }
 }
 
-__global__ void __launch_bounds__(kGjkThreads, 6) k_convex_gjk(DeviceWorld w, dyn_step_params p) {
+__global__ void __launch_bounds__(kGjkThreads) k_convex_gjk(DeviceWorld w, dyn_step_params p) {
+    __shared__ SPt simplices[kGjkGroups][4];
+    const uint32_t count = min(w.ctl[CTL_GJK_PAIRS], w.p_cap);
+    const uint32_t* list = w.np_list + (size_t)PC_COUNT * w.p_cap;
+    if (count > kGjkGroupPairs) return;  // k_convex_gjk_lanes has them
+    const Lanes<kGjkLanes> L;
+    const LaneCandidates<kGjkLanes> mine(L);
+    GjkGroup g;
+    g.s = simplices[threadIdx.x / kGjkLanes];
+    g.state = GS_IDLE;
+    for (;;) {
+        if (g.state == GS_IDLE) {
+            uint32_t ticket = 0u;
+            if (L.lane == 0u) ticket = atomicAdd(&w.ctl[CTL_GJK_NEXT], 1u);
+            ticket = L.shfl(ticket, 0u);
+            if (ticket >= count) break;
+            g.index = list[ticket];
+            DBody fb, sb;
+            WShape a, b;
+            convex_shapes(w, g.index, &a, &b, &fb, &sb);
+            g.a = group_shape(L, w, a);
+            g.b = group_shape(L, w, b);
+            g.margin = pair_margin(p, fb, sb);
+            g.tiny = 1e-4f * wmin(shape_scale(g.a), shape_scale(g.b));
+            g.count = 0u;
+            g.iter = 0u;
+            g.state = GS_FIRST;
+        }
+        f3 d;
+        if (g.state == GS_FIRST) {
+            d = g.b.center - g.a.center;
+            if (length(d) < 1e-8f) d = mk3(1.0f, 0.0f, 0.0f);
+        } else if (g.state == GS_ITER) {
+            d = -g.cl.v;
+        } else {
+            d = simplex_expand_dir(g.s, g.count);
+        }
+        const SPt sp = group_support_pair(L, g.a, g.b, d);
+        bool grown = true;  // the simplex takes the point and its closest point is wanted
+        if (g.state == GS_FIRST) {
+            // the exact centre-axis rejection of gjk_phase
+            if (dot(sp.w, d) < -(g.margin + kRejectTolerance) * length(d)) {
+                g.state = GS_IDLE;
+                grown = false;
+            }
+        } else if (g.state == GS_ITER) {
+            const f3 v = g.cl.v;
+            bool done = dot(sp.w, -v) <= dot(v, -v) + 1e-4f * wmax(1.0f, dot(v, v));
+            const bool repeats = gjk_repeats(g.cl.lam, g.count, g.s[g.count - 1u].w, sp.w);
+            if (!done) {
+                g.count = group_reduce(L, g.s, g.cl.lam);
+                done = group_holds(L, g.s, g.count, sp.w, shape_scale(g.b));
+            }
+            if (done) {
+                gjk_separated(L, w, g);
+                grown = false;
+            } else {
+                g.iter = repeats ? kGjkIterations : g.iter + 1u;
+            }
+        } else {
+            L.sync();
+            group_push(L, g.s, g.count, sp);
+            g.count += 1u;
+            if (g.count == 4u) gjk_to_epa(L, w, g);
+            grown = false;
+        }
+        if (grown) {
+            group_push(L, g.s, g.count, sp);
+            g.count += 1u;
+            g.cl = group_closest(L, mine, g.s, g.count);
+            gjk_head(L, w, g);
+        }
+        L.sync();  // the group is done with its simplex before the next pair's points replace it
+    }
+}
+
+__global__ void __launch_bounds__(kGjkThreads, 6) k_convex_gjk_lanes(DeviceWorld w, dyn_step_params p) {
     __shared__ float simplex_slices[kGjkThreads * kSimplexStride];
     const uint32_t count = min(w.ctl[CTL_GJK_PAIRS], w.p_cap);
+    if (count <= kGjkGroupPairs) return;  // k_convex_gjk has them
     const uint32_t* list = w.np_list + (size_t)PC_COUNT * w.p_cap;
     GjkLane L;
     L.s = reinterpret_cast<SPt*>(simplex_slices + threadIdx.x * kSimplexStride);
@@ -1090,6 +1237,7 @@ __global__ void __launch_bounds__(kGjkThreads, 6) k_convex_gjk(DeviceWorld w, dy
                 gjk_separated(w, L);
                 continue;
             }
+            const bool repeats = gjk_repeats(L.cl.lam, L.count, L.s[L.count - 1u].w, sp.w);
             // simplex_reduce: keep the points with weight, in order (a stable in-place compaction)
             uint32_t kc = 0;
             for (uint32_t i = 0; i < 4; ++i) {
@@ -1114,7 +1262,7 @@ __global__ void __launch_bounds__(kGjkThreads, 6) k_convex_gjk(DeviceWorld w, dy
             L.s[L.count] = sp;
             L.count += 1u;
             L.cl = simplex_closest(L.s, L.count);
-            L.iter += 1u;
+            L.iter = repeats ? kGjkIterations : L.iter + 1u;
             gjk_head(w, L);
         } else {
             L.s[L.count] = sp;
@@ -1208,7 +1356,7 @@ __global__ void __launch_bounds__(32 * kEpaWarpsPerBlock) k_convex_epa(DeviceWor
         convex_shapes(w, index, &a, &b, &fb, &sb);
         f3 simplex[4];
         for (uint32_t k = 0; k < 4; ++k) simplex[k] = xyz(w.epa_simplex[4 * (size_t)e + k]);
-        Hit hit = warp_penetrating_hit(L, w, a, b, simplex, m);
+        Hit hit = warp_penetrating_hit(L, w, group_shape(L, w, a), group_shape(L, w, b), simplex, m);
         if (L.lane == 0u) {
             if (hit.distance <= pair_margin(p, fb, sb)) push_hit(w, index, hit);
         }

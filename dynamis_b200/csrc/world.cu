@@ -81,13 +81,15 @@ struct TapeHost {
     cudaGraphExec_t back = nullptr;
 };
 
+constexpr uint32_t kForks = 5;  // fork and join events of the captured step's branches
+
 struct DeviceState {
     cudaStream_t own_stream = nullptr;
     // a second stream the captured step forks onto for kernels independent of the main line
     cudaStream_t side_stream = nullptr;
     cudaStream_t side_stream2 = nullptr;
-    cudaEvent_t fork_events[4] = {nullptr, nullptr, nullptr, nullptr};
-    cudaEvent_t join_events[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaEvent_t fork_events[kForks] = {};
+    cudaEvent_t join_events[kForks] = {};
     // the last kStepsInFlight steps' completion events: dyn_step waits for the oldest before it
     // queues another, so what the device reports (the pair demand) is at most that many steps old
     cudaEvent_t inflight[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -253,11 +255,11 @@ dyn_status ensure_device(dyn_world* w) {
         DYN_CUDA(cudaStreamCreateWithFlags(&d->own_stream, cudaStreamNonBlocking));
         DYN_CUDA(cudaStreamCreateWithFlags(&d->side_stream, cudaStreamNonBlocking));
         DYN_CUDA(cudaStreamCreateWithFlags(&d->side_stream2, cudaStreamNonBlocking));
-        for (uint32_t i = 0; i < 4; ++i) {
+        for (uint32_t i = 0; i < kForks; ++i) {
             DYN_CUDA(cudaEventCreateWithFlags(&d->fork_events[i], cudaEventDisableTiming));
             DYN_CUDA(cudaEventCreateWithFlags(&d->join_events[i], cudaEventDisableTiming));
-            DYN_CUDA(cudaEventCreateWithFlags(&d->inflight[i], cudaEventDisableTiming));
         }
+        for (uint32_t i = 0; i < 4; ++i) DYN_CUDA(cudaEventCreateWithFlags(&d->inflight[i], cudaEventDisableTiming));
         d->stream = w->user_stream ? static_cast<cudaStream_t>(w->user_stream) : d->own_stream;
         DYN_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&d->spill_host), 4 * sizeof(uint32_t), cudaHostAllocMapped));
         std::memset(d->spill_host, 0, 4 * sizeof(uint32_t));
@@ -807,7 +809,11 @@ void record_step(dyn_world* w, cudaStream_t s, uint32_t parity, bool timed, cons
     k_narrow_class<PC_BOXES><<<blocks_for(d, P, 128), 128, 0, side>>>(dw, p);
     k_convex_reject<<<blocks_for(d, P, 128), 128, 0, s>>>(dw, p);
     // persistent: lanes draw pairs from a ticket; six blocks per SM is the occupancy its registers allow
-    k_convex_gjk<<<d->sms * d->launch.gjk_blocks_per_sm, 128, 0, s>>>(dw, p);
+    // (one of the two finds the batch on its side of kGjkGroupPairs, the other returns at once)
+    fork(4, side2);
+    k_convex_gjk<<<d->sms * 4u, kGjkThreads, 0, side2>>>(dw, p);
+    k_convex_gjk_lanes<<<d->sms * d->launch.gjk_blocks_per_sm, kGjkThreads, 0, s>>>(dw, p);
+    join(4, side2);
     // separated pairs (probe) and penetrating ones (EPA) are disjoint queues
     fork(3, side2);
     k_convex_probe<<<blocks_for(d, P, 128), 128, 0, side2>>>(dw, p);
@@ -885,9 +891,10 @@ void record_step(dyn_world* w, cudaStream_t s, uint32_t parity, bool timed, cons
         }
     }
     if (world_has_ccd(w)) {
-        // continuous collision of the bodies that declare it (ccd.cuh): sweep, pick, impact, retreat
+        // continuous collision of the bodies that declare it (ccd.cuh): list, sweep, pick, impact, retreat
         mark(ST_CCD);
-        k_ccd_sweep<<<blocks_for(d, P, 128), 128, 0, s>>>(dw, p);
+        k_ccd_list<<<blocks_for(d, P, 128), 128, 0, s>>>(dw);
+        k_ccd_sweep<<<d->sms * 4u, 128, 0, s>>>(dw, p);
         k_ccd_pick<<<blocks_for(d, 2 * P, 256), 256, 0, s>>>(dw);
         k_ccd_impact<<<blocks_for(d, 2 * P, 256), 256, 0, s>>>(dw);
         k_ccd_apply<<<blocks_for(d, N, 256), 256, 0, s>>>(dw);
@@ -1146,9 +1153,11 @@ void destroy_device(dyn_world* w) {
     for (uint32_t* p : {d->sort_alt0, d->sort_alt1, d->sort_alt2}) {
         if (p) cudaFree(p);
     }
-    for (uint32_t i = 0; i < 4; ++i) {
+    for (uint32_t i = 0; i < kForks; ++i) {
         if (d->fork_events[i]) cudaEventDestroy(d->fork_events[i]);
         if (d->join_events[i]) cudaEventDestroy(d->join_events[i]);
+    }
+    for (uint32_t i = 0; i < 4; ++i) {
         if (d->inflight[i]) cudaEventDestroy(d->inflight[i]);
     }
     if (d->side_stream) cudaStreamDestroy(d->side_stream);
