@@ -252,6 +252,9 @@ struct DeviceWorld {
     const dyn_body_edit_record* edits;
     const uint4* edit_runs;
     uint32_t* edit_count;
+    // the sorts' and scans' words that start a step at zero (digit histograms, tickets, scan look-back)
+    uint32_t* step_words;
+    uint32_t step_word_count;
     // counters (reference slots) and control words
     uint32_t* counters;
     uint32_t* ctl;

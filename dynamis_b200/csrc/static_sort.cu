@@ -9,8 +9,8 @@
 // Limits and sharing:
 //   * at most DYN_STATIC_SORT_MAX_KEYS keys per call (larger n is refused with DYN_ERR_CAPACITY);
 //   * the array is shared by every call on a device and keeps the last call's contents; each call
-//     clears the parts that must start at zero (digit histograms, tile tickets, look-back words,
-//     status) on its stream before its kernels run;
+//     clears the parts that must start at zero (digit histograms, tile tickets, status, and in the
+//     histogram kernel the look-back words) on its stream before its passes run;
 //   * calls whose work overlaps on the GPU (different streams, or concurrent host threads) race
 //     on the array and must be serialised by the caller;
 //   * the array is held by every GPU that loads the library, until the process exits.
@@ -126,21 +126,20 @@ extern "C" DYN_API dyn_status dyn_radix_sort_static(uint32_t* major, uint32_t* m
     uint32_t* tickets = scratch + kTickets;
     uint32_t* status = scratch + kStatus;
     uint32_t* lookback = scratch + kLookback;
-    // what must start at zero for this call; the rest is overwritten before it is read
+    // what must start at zero for this call; the rest is overwritten before it is read (the histogram
+    // clears the look-back words)
     if (cudaMemsetAsync(hist, 0, passes * 256 * sizeof(uint32_t), s) != cudaSuccess) return DYN_ERR_CUDA;
     // the 16 tile-ticket words and the 16 status words that follow them
     if (cudaMemsetAsync(tickets, 0, 32 * sizeof(uint32_t), s) != cudaSuccess) return DYN_ERR_CUDA;
-    if (cudaMemsetAsync(lookback, 0, (size_t)passes * tiles * 256 * sizeof(uint32_t), s) != cudaSuccess) return DYN_ERR_CUDA;
     if (first_ticket) {
         // test hook only: the digit passes' tickets start above tile 0 (see dyn_debug_sort_fault)
         static const uint32_t tickets[kMaxPasses] = {1, 1, 1, 1, 1, 1, 1, 1};
         if (cudaMemcpyAsync(tickets_word(scratch), tickets, sizeof(tickets), cudaMemcpyHostToDevice, s) != cudaSuccess)
             return DYN_ERR_CUDA;
     }
-    k_sort_histogram<<<div_up(n, 256) < 592u ? div_up(n, 256) : 592u, 256, 0, s>>>(major, minor, nullptr, n, n,
-                                                                                     (int)major_digits, (int)minor_digits, hist);
-    if (cudaGetLastError() != cudaSuccess) return DYN_ERR_CUDA;
-    k_sort_offsets<<<1, 256, 0, s>>>(hist, (int)passes);
+    const SortSource src{{nullptr, nullptr, nullptr}, 1u, n, n, 0u};
+    k_sort_histogram<<<div_up(n, 256) < 592u ? div_up(n, 256) : 592u, 256, 0, s>>>(major, minor, src, (int)major_digits,
+                                                                                     (int)minor_digits, hist, lookback, tiles);
     if (cudaGetLastError() != cudaSuccess) return DYN_ERR_CUDA;
     uint32_t* src_major = major;
     uint32_t* src_minor = minor;
@@ -157,19 +156,10 @@ extern "C" DYN_API dyn_status dyn_radix_sort_static(uint32_t* major, uint32_t* m
         uint32_t* oth_in = on_minor ? src_major : src_minor;
         uint32_t* oth_out = on_minor ? dst_major : dst_minor;
         uint32_t* lb = lookback + (size_t)p * tiles * 256;
-        if (two && payload) {
-            k_onesweep<true, true><<<tiles, kSortThreads, 0, s>>>(key_in, oth_in, src_val, key_out, oth_out, dst_val, nullptr, n,
-                                                                   n, shift, hist + p * 256, lb, tickets + p, status, limit);
-        } else if (two) {
-            k_onesweep<true, false><<<tiles, kSortThreads, 0, s>>>(key_in, oth_in, nullptr, key_out, oth_out, nullptr, nullptr,
-                                                                    n, n, shift, hist + p * 256, lb, tickets + p, status, limit);
-        } else if (payload) {
-            k_onesweep<false, true><<<tiles, kSortThreads, 0, s>>>(key_in, nullptr, src_val, key_out, nullptr, dst_val, nullptr,
-                                                                    n, n, shift, hist + p * 256, lb, tickets + p, status, limit);
-        } else {
-            k_onesweep<false, false><<<tiles, kSortThreads, 0, s>>>(key_in, nullptr, nullptr, key_out, nullptr, nullptr, nullptr,
-                                                                     n, n, shift, hist + p * 256, lb, tickets + p, status, limit);
-        }
+        auto pass = two && payload ? k_onesweep<true, true> : two ? k_onesweep<true, false>
+                    : payload ? k_onesweep<false, true> : k_onesweep<false, false>;
+        pass<<<tiles, kSortThreads, 0, s>>>(key_in, oth_in, src_val, key_out, oth_out, dst_val, src, p % 2 == 0, shift,
+                                            hist + p * 256, passes, lb, tickets + p, status, limit);
         if (cudaGetLastError() != cudaSuccess) return DYN_ERR_CUDA;
         uint32_t* t;
         t = src_major; src_major = dst_major; dst_major = t;

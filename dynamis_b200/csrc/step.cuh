@@ -45,8 +45,12 @@ __device__ __forceinline__ void or_counter(uint32_t* counter, uint32_t value) {
 
 #define GRID_STRIDE(i, n) for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
 
-// Counters that persist across steps (crates/dynamis-abi/src/counter.rs: Maintained).
-__global__ void k_reset(DeviceWorld w) {
+// The step's counters and control words back to zero (those that persist across steps,
+// crates/dynamis-abi/src/counter.rs: Maintained, stay), with the sorts' and scans' words, so that none
+// of them needs a memset of its own in the graph.
+__global__ void __launch_bounds__(256) k_reset(DeviceWorld w) {
+    GRID_STRIDE(i, w.step_word_count) w.step_words[i] = 0u;
+    if (blockIdx.x != 0) return;
     for (uint32_t i = threadIdx.x; i < DYN_COUNTER_DEVICE_COUNT; i += blockDim.x) {
         if (i == DYN_COUNTER_ARCHIVED || i == DYN_COUNTER_STEP || i == DYN_COUNTER_RESTING) continue;
         w.counters[i] = 0u;

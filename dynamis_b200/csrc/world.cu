@@ -115,10 +115,8 @@ struct DeviceState {
     uint32_t* query_words = nullptr;
     uint32_t query_cap = 0, hit_cap = 0;
     // sort and scan scratch
-    uint32_t* hist = nullptr;          // 8 x 256
-    uint32_t* tile_counters = nullptr; // 16
-    uint32_t* lookback = nullptr;
-    size_t lookback_words = 0;
+    uint32_t* op_words = nullptr;  // the operator's and the queries' words (SortWords), cleared by each call
+    uint32_t* lookback = nullptr;  // the digit passes' look-back words, cleared by the histogram kernel
     uint32_t* sort_alt0 = nullptr;  // operator scratch (dyn_radix_sort)
     uint32_t* sort_alt1 = nullptr;
     uint32_t* sort_alt2 = nullptr;
@@ -181,6 +179,17 @@ dyn_status alloc(dyn_world* w, DeviceState* d, T** out, size_t count) {
     *out = static_cast<T*>(p);
     return DYN_OK;
 }
+
+// Words of the sorts and scans that must start at zero. A step's (DeviceWorld::step_words, cleared by
+// k_reset): the entry sort's and the contact sort's digit histograms and tile tickets, then the grid
+// scan's and the solver-row scan's ticket and look-back words. An operator call's or a query's
+// (DeviceState::op_words): one histogram and its tickets, then one scan's words.
+constexpr uint32_t kEntryHist = 0u, kContactHist = kMaxSegments * 4u * 256u, kStepTickets = kContactHist + 8u * 256u;
+constexpr uint32_t kStepScans = kStepTickets + 32u;
+constexpr uint32_t kOpTickets = 8u * 256u, kOpScan = kOpTickets + 16u;
+uint32_t scan_words(uint32_t cap) { return 1u + std::max((cap + kScanTile - 1u) / kScanTile, 1u); }
+// Look-back words for the longest sort: eight passes over the entries' segments or the pairs.
+size_t lookback_words(size_t keys) { return (size_t)8 * ((keys + kSortTile - 1) / kSortTile + kMaxSegments) * 256; }
 
 dyn_status alloc_contacts(dyn_world* w, DeviceState* d, ContactSet* s, uint32_t cap) {
     dyn_status st;
@@ -379,11 +388,10 @@ dyn_status ensure_device(dyn_world* w) {
         A(dw.counters, 64);
         A(dw.ctl, CTL_COUNT);
         A(d->staging, N);
-        A(d->hist, 8 * 256);
-        A(d->tile_counters, 16);
-        uint32_t max_tiles = std::max(div_up(std::max(E, P), kSortTile), 1u);
-        d->lookback_words = (size_t)8 * max_tiles * 256;
-        A(d->lookback, d->lookback_words);
+        dw.step_word_count = kStepScans + scan_words(3u * K) + scan_words(N);
+        A(dw.step_words, dw.step_word_count);
+        A(d->op_words, kOpScan + scan_words(K));
+        A(d->lookback, lookback_words(std::max(E, P)));
 #undef A
         if ((st = alloc_contacts(w, d, &dw.tmp, P))) return st;
         dw.s_cap = P;
@@ -625,27 +633,16 @@ dyn_status download_states(dyn_world* w, std::vector<dyn_body_state_record>* out
     return DYN_OK;
 }
 
-// Stable LSD sort launches on `s` (see sort.cuh). Data ends in the primary buffers.
+// Stable LSD sort launches on `s` (see sort.cuh). Data ends in the primary buffers. `hist` and
+// `tickets` start at zero. `cap` bounds the keys of all segments together.
 void record_sort(DeviceState* d, cudaStream_t s, uint32_t* major, uint32_t* minor, uint32_t* val, uint32_t* major_alt,
-                 uint32_t* minor_alt, uint32_t* val_alt, const uint32_t* count_ptr, uint32_t n_fixed, uint32_t cap,
-                 uint32_t major_digits, uint32_t minor_digits, uint32_t spin_limit = kLookbackSpinLimit,
-                 uint32_t first_ticket = 0) {
+                 uint32_t* minor_alt, uint32_t* val_alt, const SortSource& src, uint32_t cap, uint32_t major_digits,
+                 uint32_t minor_digits, uint32_t* hist, uint32_t* tickets, uint32_t spin_limit = kLookbackSpinLimit) {
     uint32_t passes = major_digits + minor_digits;
     if (passes == 0) return;
-    uint32_t tiles = std::max(div_up(cap, kSortTile), 1u);
-    cudaMemsetAsync(d->hist, 0, passes * 256 * 4, s);
-    cudaMemsetAsync(d->tile_counters, 0, 16 * 4, s);
-    if (first_ticket) {
-        // test hook only: every pass's tickets start above tile 0, so the tiles after it wait on a
-        // look-back word nothing writes until their bounded polls run out
-        static uint32_t tickets[8];
-        for (uint32_t& t : tickets) t = first_ticket;
-        cudaMemcpyAsync(d->tile_counters, tickets, sizeof(tickets), cudaMemcpyHostToDevice, s);
-    }
-    cudaMemsetAsync(d->lookback, 0, (size_t)passes * tiles * 256 * 4, s);
-    k_sort_histogram<<<std::min(div_up(cap, 256), d->sms * 4u), 256, 0, s>>>(major, minor, count_ptr, n_fixed, cap,
-                                                                            (int)major_digits, (int)minor_digits, d->hist);
-    k_sort_offsets<<<1, 256, 0, s>>>(d->hist, (int)passes);
+    const uint32_t tiles = sort_tickets(cap, src.segments);
+    k_sort_histogram<<<std::min(div_up(cap, 256), d->sms * 4u), 256, 0, s>>>(major, minor, src, (int)major_digits,
+                                                                            (int)minor_digits, hist, d->lookback, tiles);
     uint32_t* src_major = major;
     uint32_t* src_minor = minor;
     uint32_t* src_val = val;
@@ -653,6 +650,8 @@ void record_sort(DeviceState* d, cudaStream_t s, uint32_t* major, uint32_t* mino
     uint32_t* dst_minor = minor_alt;
     uint32_t* dst_val = val_alt;
     bool two = minor != nullptr;
+    auto pass = two && val ? k_onesweep<true, true> : two ? k_onesweep<true, false>
+                : val ? k_onesweep<false, true> : k_onesweep<false, false>;
     for (uint32_t p = 0; p < passes; ++p) {
         bool on_minor = p < minor_digits;
         int shift = 8 * (int)(on_minor ? p : p - minor_digits);
@@ -660,44 +659,30 @@ void record_sort(DeviceState* d, cudaStream_t s, uint32_t* major, uint32_t* mino
         uint32_t* key_out = on_minor ? dst_minor : dst_major;
         uint32_t* oth_in = on_minor ? src_major : src_minor;
         uint32_t* oth_out = on_minor ? dst_major : dst_minor;
-        uint32_t* lb = d->lookback + (size_t)p * tiles * 256;
-        uint32_t* status = d->dw.ctl + CTL_STATUS;
-        if (two && val) {
-            k_onesweep<true, true><<<tiles, kSortThreads, 0, s>>>(key_in, oth_in, src_val, key_out, oth_out, dst_val, count_ptr,
-                                                                   n_fixed, cap, shift, d->hist + p * 256, lb,
-                                                                   d->tile_counters + p, status, spin_limit);
-        } else if (two) {
-            k_onesweep<true, false><<<tiles, kSortThreads, 0, s>>>(key_in, oth_in, nullptr, key_out, oth_out, nullptr, count_ptr,
-                                                                    n_fixed, cap, shift, d->hist + p * 256, lb,
-                                                                    d->tile_counters + p, status, spin_limit);
-        } else if (val) {
-            k_onesweep<false, true><<<tiles, kSortThreads, 0, s>>>(key_in, nullptr, src_val, key_out, nullptr, dst_val, count_ptr,
-                                                                    n_fixed, cap, shift, d->hist + p * 256, lb,
-                                                                    d->tile_counters + p, status, spin_limit);
-        } else {
-            k_onesweep<false, false><<<tiles, kSortThreads, 0, s>>>(key_in, nullptr, nullptr, key_out, nullptr, nullptr,
-                                                                     count_ptr, n_fixed, cap, shift, d->hist + p * 256, lb,
-                                                                     d->tile_counters + p, status, spin_limit);
-        }
+        pass<<<tiles, kSortThreads, 0, s>>>(key_in, oth_in, src_val, key_out, oth_out, dst_val, src, p % 2 == 0, shift,
+                                            hist + p * 256, passes, d->lookback + (size_t)p * tiles * 256, tickets + p,
+                                            d->dw.ctl + CTL_STATUS, spin_limit);
         std::swap(src_major, dst_major);
         std::swap(src_minor, dst_minor);
         std::swap(src_val, dst_val);
     }
     if (passes % 2 == 1) {
-        // odd pass count: results sit in the alternate buffers
+        // odd pass count: results sit in the alternate buffers (one segment: packed at their start)
         size_t bytes = (size_t)cap * 4;
         cudaMemcpyAsync(major, src_major, bytes, cudaMemcpyDeviceToDevice, s);
         if (two) cudaMemcpyAsync(minor, src_minor, bytes, cudaMemcpyDeviceToDevice, s);
         if (val) cudaMemcpyAsync(val, src_val, bytes, cudaMemcpyDeviceToDevice, s);
     }
 }
+SortSource one_segment(const uint32_t* count_ptr, uint32_t n_fixed, uint32_t cap) {
+    return SortSource{{count_ptr, nullptr, nullptr}, 1u, n_fixed, cap, 0u};
+}
 
+// `words`: the scan's ticket and look-back words, at zero (scan_words(cap) of them).
 void record_scan(DeviceState* d, cudaStream_t s, const uint32_t* in, uint32_t* out, const uint32_t* count_ptr,
-                 uint32_t n_fixed, uint32_t cap, uint32_t* total) {
-    uint32_t tiles = std::max(div_up(cap, kSortTile), 1u);
-    cudaMemsetAsync(d->tile_counters + 15, 0, 4, s);
-    cudaMemsetAsync(d->lookback, 0, (size_t)tiles * 4, s);
-    k_scan_exclusive<<<tiles, kSortThreads, 0, s>>>(in, out, count_ptr, n_fixed, cap, total, d->lookback, d->tile_counters + 15,
+                 uint32_t n_fixed, uint32_t cap, uint32_t* total, uint32_t* words) {
+    uint32_t tiles = std::max(div_up(cap, kScanTile), 1u);
+    k_scan_exclusive<<<tiles, kScanThreads, 0, s>>>(in, out, count_ptr, n_fixed, cap, total, words + 1, words,
                                                     d->dw.ctl + CTL_STATUS, kLookbackSpinLimit);
 }
 
@@ -749,7 +734,7 @@ void record_step(dyn_world* w, cudaStream_t s, uint32_t parity, bool timed, cons
     dw.rest_out = d->rest_ids[1u - parity];
     dw.rest_out_slots = d->rest_slots[1u - parity];
     mark(ST_BEGIN);
-    k_reset<<<1, 64, 0, s>>>(dw);
+    k_reset<<<blocks_for(d, dw.step_word_count, 256), 256, 0, s>>>(dw);
     if (dw.jcount) k_joint_count<<<blocks_for(d, std::max(dw.jfilter_count, 1u), 256), 256, 0, s>>>(dw);
     if (d->edit_graphs) {
         k_clear_inputs<<<blocks_for(d, N, 256), 256, 0, s>>>(dw);
@@ -766,16 +751,15 @@ void record_step(dyn_world* w, cudaStream_t s, uint32_t parity, bool timed, cons
     k_entry_count<true><<<blocks_for(d, K, 256), 256, 0, s>>>(dw);
     // one scan over the three runs' counts back to back; each run's key positions are its offsets
     // less the offset at the start of its third
-    record_scan(d, s, dw.run_count, dw.run_offset, nullptr, 3 * dw.k, 3 * K, dw.held + HELD_SCRATCH);
+    record_scan(d, s, dw.run_count, dw.run_offset, nullptr, 3 * dw.k, 3 * K, dw.held + HELD_SCRATCH,
+                dw.step_words + kStepScans);
     k_grid_gate<<<1, 32, 0, s>>>(dw);
     k_entry_emit<true><<<blocks_for(d, K, 256), 256, 0, s>>>(dw);
     mark(ST_ENTRY_SORT);
-    for (uint32_t run = 0; run < 3; ++run) {
-        const uint32_t* count = dw.held + (run == RUN_AWAKE ? HELD_AWAKE
-                                           : run == RUN_IMMOVABLE ? HELD_SORT_IMMOVABLE : HELD_SORT_RESTING);
-        record_sort(d, s, dw.run_key + (size_t)run * E, nullptr, dw.run_val + (size_t)run * E, dw.ekey_alt, nullptr,
-                    dw.eval_alt, count, 0, E, 4, 0);
-    }
+    // the three runs' sorts in the same launches; a kept run's segment holds no key
+    const SortSource runs{{dw.held + HELD_AWAKE, dw.held + HELD_SORT_IMMOVABLE, dw.held + HELD_SORT_RESTING}, 3u, 0u, E, E};
+    record_sort(d, s, dw.run_key, nullptr, dw.run_val, dw.ekey_alt, nullptr, dw.eval_alt, runs, E, 4, 0, dw.step_words + kEntryHist,
+                dw.step_words + kStepTickets);
     k_entry_merge<<<blocks_for(d, E, 256), 256, 0, s>>>(dw);
     mark(ST_PAIRS);
     k_cell_clear<<<blocks_for(d, 1u << dw.cell_bits, 256), 256, 0, s>>>(dw);
@@ -824,8 +808,9 @@ void record_step(dyn_world* w, cudaStream_t s, uint32_t parity, bool timed, cons
     mark(ST_COMPACT);
     k_contact_keys<<<blocks_for(d, C, 256), 256, 0, s>>>(dw);
     const uint32_t words = key_words(std::max(dw.k, 1u));
-    record_sort(d, s, dw.cmaj, dw.cmin, dw.cval, dw.cmaj_alt, dw.cmin_alt, dw.cval_alt, dw.ctl + CTL_STAGED, 0, dw.s_cap, words,
-                words);
+    record_sort(d, s, dw.cmaj, dw.cmin, dw.cval, dw.cmaj_alt, dw.cmin_alt, dw.cval_alt,
+                one_segment(dw.ctl + CTL_STAGED, 0, dw.s_cap), dw.s_cap, words, words, dw.step_words + kContactHist,
+                dw.step_words + kStepTickets + 16u);
     k_contact_gather<<<blocks_for(d, C, 128), 128, 0, s>>>(dw);
     // the solver blocks (target speeds, row claims) beside the identity, islands and wake passes:
     // neither reads what the other writes (the relay rewrites only the w word of a contact's rows
@@ -833,7 +818,8 @@ void record_step(dyn_world* w, cudaStream_t s, uint32_t parity, bool timed, cons
     mark(ST_SOLVER_PREPARE);
     fork(2, side);
     k_solver_blocks<<<blocks_for(d, C, 256), 256, 0, side>>>(dw, p);
-    record_scan(d, side, dw.row_flag, dw.row_offset, nullptr, std::max(dw.n, 1u), N, dw.ctl + CTL_SOLVER_ROWS);
+    record_scan(d, side, dw.row_flag, dw.row_offset, nullptr, std::max(dw.n, 1u), N, dw.ctl + CTL_SOLVER_ROWS,
+                dw.step_words + kStepScans + scan_words(3u * d->k_cap));
     k_solver_row_list<<<blocks_for(d, N, 256), 256, 0, side>>>(dw);
     mark(ST_IDENTITY);
     if (tape) k_tape_clear_relay<<<blocks_for(d, 4 * C, 256), 256, 0, s>>>(*tape);
@@ -1330,7 +1316,7 @@ dyn_status widen_pair_stream(dyn_world* w) {
                      {reinterpret_cast<void**>(&dw.cmin_alt), P * sizeof(uint32_t), nullptr},
                      {reinterpret_cast<void**>(&dw.cval_alt), P * sizeof(uint32_t), nullptr},
                      {reinterpret_cast<void**>(&d->lookback),
-                      (size_t)8 * std::max(div_up(std::max<size_t>(d->e_cap, P), kSortTile), 1u) * 256 * sizeof(uint32_t), nullptr}};
+                      lookback_words(std::max<size_t>(d->e_cap, P)) * sizeof(uint32_t), nullptr}};
     for (Buffer& b : list) {
         if (cudaMalloc(&b.fresh, b.bytes) != cudaSuccess) {
             for (Buffer& f : list) if (f.fresh) cudaFree(f.fresh);
@@ -1347,7 +1333,6 @@ dyn_status widen_pair_stream(dyn_world* w) {
         *b.slot = b.fresh;
     }
     d->p_cap = dw.p_cap = dw.s_cap = (uint32_t)P;
-    d->lookback_words = (size_t)8 * std::max(div_up(std::max<size_t>(d->e_cap, P), kSortTile), 1u) * 256;
     release_graphs(d);  // the graphs hold the old buffers and capacity
     return DYN_OK;
 }
@@ -2429,11 +2414,13 @@ DYN_API dyn_status dyn_query(dyn_world* w, dyn_query_record* queries, uint32_t n
     DYN_CUDA(cudaMemsetAsync(d->query_words, 0, (64 + CTL_COUNT) * sizeof(uint32_t), s));
     // the query's grid takes the merged list, cell table and run extents: the next step lists again
     DYN_CUDA(cudaMemsetAsync(d->dw.held + HELD_LIST_KEPT, 0, 2 * sizeof(uint32_t), s));
+    DYN_CUDA(cudaMemsetAsync(d->op_words, 0, (kOpScan + scan_words(K)) * sizeof(uint32_t), s));
     k_aabb<<<blocks_for(d, K, 128), 128, 0, s>>>(dw, p);
     k_entry_count<false><<<blocks_for(d, K, 256), 256, 0, s>>>(dw);
-    record_scan(d, s, dw.entry_count, dw.entry_offset, nullptr, dw.k, K, dw.ctl + CTL_ENTRIES);
+    record_scan(d, s, dw.entry_count, dw.entry_offset, nullptr, dw.k, K, dw.ctl + CTL_ENTRIES, d->op_words + kOpScan);
     k_entry_emit<false><<<blocks_for(d, K, 256), 256, 0, s>>>(dw);
-    record_sort(d, s, dw.ekey, nullptr, dw.eval, dw.ekey_alt, nullptr, dw.eval_alt, dw.ctl + CTL_ENTRIES, 0, E, 4, 0);
+    record_sort(d, s, dw.ekey, nullptr, dw.eval, dw.ekey_alt, nullptr, dw.eval_alt,
+                one_segment(dw.ctl + CTL_ENTRIES, 0, E), E, 4, 0, d->op_words, d->op_words + kOpTickets);
     k_cell_clear<<<blocks_for(d, 1u << dw.cell_bits, 256), 256, 0, s>>>(dw);
     k_cell_insert<<<blocks_for(d, E, 256), 256, 0, s>>>(dw);
     DYN_CUDA(cudaMemcpyAsync(d->query_buf, queries, (size_t)n * sizeof(dyn_query_record), cudaMemcpyHostToDevice, s));
@@ -2751,15 +2738,25 @@ DYN_API dyn_status dyn_radix_sort(dyn_world* w, uint32_t* major, uint32_t* minor
         DYN_CUDA(cudaMalloc(&d->sort_alt2, (size_t)n * 4));
         d->sort_alt_cap = n;
     }
-    uint32_t tiles = div_up(n, kSortTile);
-    if ((size_t)(major_digits + minor_digits) * tiles * 256 > d->lookback_words) {
+    // the refusal counts tiles of 2048 keys, whatever the passes use
+    auto tiles_of = [](size_t keys) { return std::max<size_t>((keys + 2047u) / 2048u, 1u); };
+    if ((size_t)(major_digits + minor_digits) * tiles_of(n) > 8 * tiles_of(std::max(d->e_cap, d->p_cap))) {
         return fail(w, DYN_ERR_CAPACITY, "dyn_radix_sort: more keys than the world's sort scratch holds");
     }
     const uint32_t limit = d->sort_fault_armed ? d->sort_fault_limit : kLookbackSpinLimit;
     const uint32_t first_ticket = d->sort_fault_armed ? d->sort_fault_skip : 0u;
     d->sort_fault_armed = false;
+    DYN_CUDA(cudaMemsetAsync(d->op_words, 0, kOpScan * sizeof(uint32_t), d->stream));
+    if (first_ticket) {
+        // test hook only: every pass's tickets start above tile 0, so the tiles after it wait on a
+        // look-back word nothing writes until their bounded polls run out
+        static uint32_t tickets[8];
+        for (uint32_t& t : tickets) t = first_ticket;
+        DYN_CUDA(cudaMemcpyAsync(d->op_words + kOpTickets, tickets, sizeof(tickets), cudaMemcpyHostToDevice, d->stream));
+    }
     record_sort(d, d->stream, major, minor, payload, d->sort_alt0, minor ? d->sort_alt1 : nullptr,
-                payload ? d->sort_alt2 : nullptr, nullptr, n, n, major_digits, minor_digits, limit, first_ticket);
+                payload ? d->sort_alt2 : nullptr, one_segment(nullptr, n, n), n, major_digits, minor_digits, d->op_words,
+                d->op_words + kOpTickets, limit);
     DYN_CUDA(cudaGetLastError());
     return DYN_OK;
 }
