@@ -246,6 +246,11 @@ struct DeviceWorld {
     uint2* jlayers;     // (first entry of jrows, count)
     uint2* jcomps;      // (first layer, layer count)
     uint4* jgroups;     // warp groups: first component, components, lanes each, deepest stack
+    // the joints in solve order (k_joint_prepare, once per substep)
+    uint4* jo_meta;     // joint, first row, second row, flags
+    float4* jo_mass;    // the three rows' masses
+    float4* jo_arm;     // [2 per joint] a side's arm, inverse mass (0 when inert)
+    float4* jo_anchor;  // [2 per joint] a side's anchor, break limit
     uint2* jfilter;     // sorted (lower row, higher row) of the joints that disable collisions
     uint32_t* jfilter_joint;
     // queued body edits of this step (runs of one row each; *edit_count runs)

@@ -476,6 +476,10 @@ dyn_status upload_joints(dyn_world* w) {
     JA(jlayers, plan.layers.size() * 4);
     JA(jcomps, plan.components.size() * 4);
     JA(jgroups, plan.groups.size() * 4);
+    JA(jo_meta, m * sizeof(uint4));
+    JA(jo_mass, m * sizeof(float4));
+    JA(jo_arm, 2 * (size_t)m * sizeof(float4));
+    JA(jo_anchor, 2 * (size_t)m * sizeof(float4));
     JA(jfilter, fpairs.size() * sizeof(uint2));
     JA(jfilter_joint, fjoint.size() * 4);
 #undef JA
@@ -841,6 +845,7 @@ void record_step(dyn_world* w, cudaStream_t s, uint32_t parity, bool timed, cons
         k_integrate<<<blocks_for(d, N, 256), 256, 0, s>>>(dw, p);
         const uint32_t st = d->launch.solve_threads;
         k_solve_prepare<<<blocks_for(d, C, st), st, 0, s>>>(dw, sub == 0u);
+        if (joint_blocks) k_joint_prepare<<<blocks_for(d, dw.jcount, 128), 128, 0, s>>>(dw);
         if (sub == 0) {
             mark(ST_WARM);
             if (joint_blocks) k_joints<JP_WARM><<<joint_blocks, 32, 0, s>>>(dw, p);
