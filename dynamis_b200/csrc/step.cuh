@@ -651,7 +651,14 @@ __device__ __forceinline__ uint32_t cell_find(const DeviceWorld& w, uint32_t liv
 // The coarse links spread over gridDim.y: thread (i, y) walks collider i's cells at the occupied
 // levels whose rank among the occupied levels is y, y + gridDim.y, ... (the walk of one collider is
 // a chain of dependent lookups; splitting it by level shortens the chain a thread waits through).
+// With gridDim.z = 8 a thread walks one of the at most eight cells of a level (the one whose offsets
+// from the lowest are the bits of blockIdx.z), which shortens it again. The repeated loads and checks
+// of the entry cost more than that saves once the threads fill the chip (262,144 bodies), so the
+// split is by the collider count: up to kCoarseSplitColliders sixteen level slices and eight cells,
+// above it four and all cells.
 constexpr uint32_t kCoarseLevelSlices = 4u;
+constexpr uint32_t kCoarseSplitColliders = 8192u;
+constexpr uint32_t kCoarseSplitSlices = 16u, kCoarseSplitCells = 8u;
 constexpr uint32_t kRunBatch = 4u;            // entries of a cell run the coarse walk loads together
 constexpr uint32_t kCellBatch = 2u;           // the same for the same-cell scan, whose runs are short
 constexpr uint32_t kNoEntry = 0xFFFFFFFFu;
@@ -686,8 +693,15 @@ __global__ void __launch_bounds__(128) k_pairs_coarse(DeviceWorld w) {
             // span only comes from a non-finite box, whose walk is cut short and counted.
             if ((long long)hi.x - lo.x > 3 || (long long)hi.y - lo.y > 3 || (long long)hi.z - lo.z > 3 || hi.x < lo.x ||
                 hi.y < lo.y || hi.z < lo.z) {
-                add_counter(&w.counters[DYN_COUNTER_ENTRY_FAULTS], 1u);
+                if (blockIdx.z == 0u) add_counter(&w.counters[DYN_COUNTER_ENTRY_FAULTS], 1u);
                 continue;
+            }
+            const bool split = gridDim.z > 1u;
+            if (split) {  // one cell; a span of more than two (a box at the check's edge) falls to the last octants
+                const int ox = (int)(blockIdx.z & 1u), oy = (int)((blockIdx.z >> 1) & 1u), oz = (int)(blockIdx.z >> 2);
+                if (lo.x + ox > hi.x || lo.y + oy > hi.y || lo.z + oz > hi.z) continue;
+                lo = I3{lo.x + ox, lo.y + oy, lo.z + oz};
+                hi = I3{ox ? hi.x : lo.x, oy ? hi.y : lo.y, oz ? hi.z : lo.z};
             }
             for (int x = lo.x; x <= hi.x; ++x)
                 for (int y = lo.y; y <= hi.y; ++y)

@@ -786,7 +786,9 @@ void record_step(dyn_world* w, cudaStream_t s, uint32_t parity, bool timed, cons
         cudaStreamWaitEvent(s, d->join_events[k], 0);
     };
     fork(0, side);
-    k_pairs_coarse<<<dim3(blocks_for(d, K, 128), kCoarseLevelSlices), 128, 0, s>>>(dw);
+    const dim3 coarse_grid = K <= kCoarseSplitColliders ? dim3(blocks_for(d, K, 128), kCoarseSplitSlices, kCoarseSplitCells)
+                                                        : dim3(blocks_for(d, K, 128), kCoarseLevelSlices);
+    k_pairs_coarse<<<coarse_grid, 128, 0, s>>>(dw);
     k_pairs_cell<<<blocks_for(d, E, 256), 256, 0, side>>>(dw);
     join(0, side);
     // the candidate pairs stay in emission order; the contacts are sorted into pair order below
