@@ -77,6 +77,7 @@ enum Ctl : uint32_t {
     CTL_REST_NEXT = 23,      // frozen contacts this step's commit wrote
     CTL_CCD_SWEEPS = 24,     // directions of pairs the continuous-collision pass sweeps
     CTL_CCD_NEXT = 25,       // the next of them
+    CTL_BOX_HITS = 26,       // touching box pairs queued for the manifold
     CTL_COUNT = 32
 };
 
@@ -213,6 +214,8 @@ struct DeviceWorld {
     float4* epa_simplex;     // [4][slot]: the GJK simplex (w.xyz) EPA starts from
     uint32_t* probe_list;    // pair indices of separated convex pairs
     float4* probe_data;      // [6][slot]: their simplex, point count, distance, closest points, normal
+    uint32_t* box_hits;      // pair indices of touching box pairs
+    float4* box_axis;        // [2][slot]: their axis + depth, face depth + code (BoxAxis)
     uint32_t* hit_list;      // pair indices of convex hits
     float4* hit_data;        // [2][slot]: point.xyz + distance, normal.xyz
     ContactSet cur;  // this step's contacts in sorted pair order

@@ -434,13 +434,15 @@ __device__ uint32_t clip_polygon(const f3* pts, const uint32_t* ids, uint32_t co
     return oc;
 }
 
-// narrowphase.wgsl:325-473
-__device__ Mani box_box_sat(const DBody& fb, const DColl& fc, const DBody& sb, const DColl& sc, float margin) {
-    Mani m;
-    m.count = 0;
-    m.normal = s3(0.0f);
-    BoxGeo L = box_geo(fb, fc);
-    BoxGeo R = box_geo(sb, sc);
+// narrowphase.wgsl:325-473 in two parts: which axis answers the pair, if any (most of a pile's box pairs
+// end here, with every thread of a warp on the same axes), and the manifold on that axis.
+struct BoxAxis {
+    f3 axis;
+    float depth, face_depth;
+    uint32_t code;  // the face's box (1: the second's) or kBoxEdge | first edge << 2 | second edge
+};
+constexpr uint32_t kBoxEdge = 16u;
+__device__ __forceinline__ bool box_box_axis(const BoxGeo& L, const BoxGeo& R, float margin, BoxAxis* out) {
     f3 delta = R.center - L.center;
     float face_depth = 1e30f;
     f3 face_axis = L.axes[0];
@@ -464,7 +466,7 @@ __device__ Mani box_box_sat(const DBody& fb, const DColl& fc, const DBody& sb, c
     // No contact whatever the edge axes give: an edge axis wins only when its depth is below the face
     // depth (edge_depth <= edge_depth + 1e-3 * extent < face_depth, rounding being monotone), and
     // either depth at or below -margin answers no contact below. So the nine edge axes are skipped.
-    if (face_depth <= -margin) return m;
+    if (face_depth <= -margin) return false;
     float edge_depth = 1e30f;
     f3 edge_axis = face_axis;
     uint32_t efa = 0, esa = 0;
@@ -485,16 +487,24 @@ __device__ Mani box_box_sat(const DBody& fb, const DColl& fc, const DBody& sb, c
     }
     float extent = wmax(wmax(L.half.x, L.half.y), L.half.z) + wmax(wmax(R.half.x, R.half.y), R.half.z);
     bool edge_sep = edge_depth + 1e-3f * extent < face_depth;
-    float depth = edge_sep ? edge_depth : face_depth;
-    if (depth <= -margin) return m;
-    f3 axis = edge_sep ? edge_axis : face_axis;
-    f3 sgn = dot(axis, delta) < 0.0f ? -axis : axis;
+    out->depth = edge_sep ? edge_depth : face_depth;
+    out->face_depth = face_depth;
+    out->axis = edge_sep ? edge_axis : face_axis;
+    out->code = edge_sep ? (kBoxEdge | (efa << 2) | esa) : (face_on_right ? 1u : 0u);
+    return !(out->depth <= -margin);
+}
+__device__ __forceinline__ Mani box_box_manifold(const BoxGeo& L, const BoxGeo& R, const BoxAxis& found, float margin) {
+    Mani m;
+    f3 delta = R.center - L.center;
+    f3 sgn = dot(found.axis, delta) < 0.0f ? -found.axis : found.axis;
     mani_emit(&m, sgn);
-    if (edge_sep) {
+    if (found.code & kBoxEdge) {
         f3 point = (box_support_geo(L, sgn) + box_support_geo(R, -sgn)) * 0.5f;
-        mani_push(&m, point, depth, feature_pair(kFeatEdge, efa, esa));
+        mani_push(&m, point, found.depth, feature_pair(kFeatEdge, (found.code >> 2) & 3u, found.code & 3u));
         return m;
     }
+    const bool face_on_right = (found.code & 1u) != 0u;
+    const float face_depth = found.face_depth;
     const BoxGeo& ref = face_on_right ? R : L;
     const BoxGeo& inc = face_on_right ? L : R;
     f3 ref_normal = face_on_right ? -sgn : sgn;

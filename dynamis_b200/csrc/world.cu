@@ -355,6 +355,8 @@ dyn_status ensure_device(dyn_world* w) {
         A(dw.epa_simplex, 4 * (size_t)P);
         A(dw.probe_list, P);
         A(dw.probe_data, 6 * (size_t)P);
+        A(dw.box_hits, P);
+        A(dw.box_axis, 2 * (size_t)P);
         A(dw.hit_list, P);
         A(dw.hit_data, 2 * (size_t)P);
         A(dw.matched, C);
@@ -796,6 +798,7 @@ void record_step(dyn_world* w, cudaStream_t s, uint32_t parity, bool timed, cons
     k_pair_class<<<blocks_for(d, P, 256), 256, 0, s>>>(dw);
     fork(1, side);
     k_narrow_class<PC_ANALYTIC><<<blocks_for(d, P, 128), 128, 0, side>>>(dw, p);
+    k_boxes_axis<<<blocks_for(d, P, 128), 128, 0, side>>>(dw, p);
     k_narrow_class<PC_BOXES><<<blocks_for(d, P, 128), 128, 0, side>>>(dw, p);
     k_convex_reject<<<blocks_for(d, P, 128), 128, 0, s>>>(dw, p);
     // persistent: lanes draw pairs from a ticket; six blocks per SM is the occupancy its registers allow
@@ -1303,6 +1306,8 @@ dyn_status widen_pair_stream(dyn_world* w) {
                      {reinterpret_cast<void**>(&dw.epa_simplex), 4 * P * sizeof(float4), nullptr},
                      {reinterpret_cast<void**>(&dw.probe_list), P * sizeof(uint32_t), nullptr},
                      {reinterpret_cast<void**>(&dw.probe_data), 6 * P * sizeof(float4), nullptr},
+                     {reinterpret_cast<void**>(&dw.box_hits), P * sizeof(uint32_t), nullptr},
+                     {reinterpret_cast<void**>(&dw.box_axis), 2 * P * sizeof(float4), nullptr},
                      {reinterpret_cast<void**>(&dw.hit_list), P * sizeof(uint32_t), nullptr},
                      {reinterpret_cast<void**>(&dw.hit_data), 2 * P * sizeof(float4), nullptr},
                      // the staging set of the narrowphase's contacts (one per pair at most) and its sort
