@@ -156,13 +156,40 @@ __device__ SweepHit rigid_sweep(const SweepLanes& L, const DeviceWorld& w, const
     return none;
 }
 
+// Can this direction be answered "no hit" without a search? The gap along the centre axis at the
+// sweep's start bounds the distance the search would report from below (narrow.cuh, gjk_phase), and the
+// approach it is divided by is at most the relative travel plus the turning of both shapes. When the
+// gap exceeds that by more than rounding, the first step of rigid_sweep passes the end of the step
+// whatever its normal. Planes are left to the sweep, whose gap to them is one support evaluation.
+constexpr float kSweepRejectTolerance = 1e-3f;
+__device__ __forceinline__ bool sweep_cannot_reach(const DeviceWorld& w, const SweptBody& moving, const DColl& mc,
+                                                   const SweptBody& other, const DColl& oc) {
+    if (mc.kind == DYN_SHAPE_PLANE || oc.kind == DYN_SHAPE_PLANE) return false;
+    if (shape_world_geometry(mc.kind) || shape_world_geometry(oc.kind)) return false;
+    const bool other_movable = moves(other.body.inverse_mass, other.body.flags);
+    float reach = sweep_reach(w, moving, mc).spin;
+    f3 travel = moving.body.position - moving.prev_position;
+    if (other_movable) {
+        reach = reach + sweep_reach(w, other, oc).spin;
+        travel = travel - (other.body.position - other.prev_position);
+    }
+    reach = reach + length(travel);
+    const WShape free = swept_shape(moving, mc, 0.0f);
+    const WShape fixed = other_movable ? swept_shape(other, oc, 0.0f)
+                                       : world_shape(other.body.position, other.body.orientation, oc);
+    const f3 axis = fixed.center - free.center;
+    const float gap = -dot(support(w, free, axis) - support(w, fixed, -axis), axis);
+    return gap > (reach * (1.0f + kSweepRejectTolerance) + kSweepRejectTolerance) * length(axis);
+}
+
 // ccd_sweep.wgsl:188-211 (the pairs are unique, so the sorted list's duplicate check has nothing to
 // skip): the directions to sweep, as pair index * 2 + (1: the second body moves), in the class lists
 // of the narrowphase, which nothing reads after it.
 __global__ void __launch_bounds__(128) k_ccd_list(DeviceWorld w) {
     const uint32_t pairs = min(w.counters[DYN_COUNTER_PAIRS], w.p_cap);
     GRID_STRIDE(index, pairs) {
-        const uint4 f = w.c_class[w.pmaj[index]], s = w.c_class[w.pmin[index]];
+        const uint32_t fs = w.pmaj[index], ss = w.pmin[index];
+        const uint4 f = w.c_class[fs], s = w.c_class[ss];
         const uint32_t fr = f.x, sr = s.x;
         if (fr == DYN_NO_BODY || sr == DYN_NO_BODY || fr == sr) continue;
         // only a body that declares CCD sweeps (rigid_sweep's first test)
@@ -172,8 +199,14 @@ __global__ void __launch_bounds__(128) k_ccd_list(DeviceWorld w) {
         if ((f.w & 0xffu) == 0u || (s.w & 0xffu) == 0u) continue;     // SHAPE_NONE
         if (!((f.y & s.z) != 0u && (s.y & f.z) != 0u)) continue;      // collision filters
         if (joined_by_joint(w, fr, sr)) continue;
-        if (first) w.np_list[append_slot(&w.ctl[CTL_CCD_SWEEPS])] = 2u * index;
-        if (second) w.np_list[append_slot(&w.ctl[CTL_CCD_SWEEPS])] = 2u * index + 1u;
+        const SweptBody fb = load_swept(w, fr), sb = load_swept(w, sr);
+        const DColl fc = load_dcoll(w, fs), sc = load_dcoll(w, ss);
+#pragma unroll 1
+        for (uint32_t side = 0; side < 2u; ++side) {
+            if (!(side ? second : first)) continue;
+            if (side ? sweep_cannot_reach(w, sb, sc, fb, fc) : sweep_cannot_reach(w, fb, fc, sb, sc)) continue;
+            w.np_list[append_slot(&w.ctl[CTL_CCD_SWEEPS])] = 2u * index + side;
+        }
     }
 }
 
