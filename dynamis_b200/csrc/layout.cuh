@@ -78,6 +78,8 @@ enum Ctl : uint32_t {
     CTL_CCD_SWEEPS = 24,     // directions of pairs the continuous-collision pass sweeps
     CTL_CCD_NEXT = 25,       // the next of them
     CTL_BOX_HITS = 26,       // touching box pairs queued for the manifold
+    CTL_QUERY_NEXT = 27,     // a query batch's next query (in the query's own control words)
+    CTL_QUERY_LARGE = 28,    // its queries left to k_scene_query_large
     CTL_COUNT = 32
 };
 

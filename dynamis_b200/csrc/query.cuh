@@ -2,7 +2,7 @@
 // convex sweeps against the colliders (crates/dynamis-shader/shaders/scene_cast.wgsl:1-534 for the
 // candidate walk and the hit selection; scene.wgsl:1-258, 259-320, 813-873 for the hit tests).
 //
-// One block per query. The candidates are the colliders with an entry in the grid cells the
+// One warp per query, or one block where a warp cannot hold its candidates. They are the colliders with an entry in the grid cells the
 // query's box covers, level by level (grid_index.wgsl:289-388: a level whose cells under the box
 // number more than GRID_WALK_CELLS is scanned whole, entries tested against the box; otherwise its
 // cells are looked up one by one), at most QUERY_CANDIDATES of them (more set the overflow flag).
@@ -413,8 +413,10 @@ __device__ QHit shape_sweep(const DeviceWorld& w, const WShape& moving, const WS
     return q_no_hit();
 }
 
-// resolve_hit (scene_cast.wgsl:384-432) of one collider
-__device__ QHit resolve_hit(const DeviceWorld& w, const dyn_query_record& q, const WShape& world) {
+// resolve_hit (scene_cast.wgsl:384-432) of one collider. Without `whole` only the distance is wanted
+// (the selection's first pass over the candidates): a sphere or point query then leaves out the walk
+// over a hull's triangles that gives its normal, which a miss never needs either.
+__device__ QHit resolve_hit(const DeviceWorld& w, const dyn_query_record& q, const WShape& world, bool whole) {
     const uint32_t kind = q.kind;
     if (kind == DYN_QUERY_RAY) {
         const f3 direction = normalize(q_direction(q));
@@ -430,9 +432,12 @@ __device__ QHit resolve_hit(const DeviceWorld& w, const dyn_query_record& q, con
     }
     f3 normal = s3(0.0f);
     if (kind == DYN_QUERY_SPHERE || kind == DYN_QUERY_POINT) {
-        const float from_hit = overlap_hit(w, q, world, &normal);
-        const float from_geom = overlap_world_geom(w, q, world, &normal);
-        const float separation = world_geom ? from_geom : from_hit;
+        float separation = world_geom ? 0.0f : overlap_hit(w, q, world, &normal);
+        if (world_geom) {
+            separation = overlap_world_geom(w, q, world, &normal);
+        } else if (whole && separation < kQNoHit) {
+            overlap_world_geom(w, q, world, &normal);
+        }
         if (separation < kQNoHit) return QHit{separation, world.center, normal, DYN_NO_TRIANGLE};
         return q_no_hit();
     }
@@ -533,12 +538,225 @@ __device__ __forceinline__ void push_candidate(QueryShared& sh, uint32_t slot) {
     sh.candidates[at] = slot;
 }
 
-// One block per query (scene_cast.wgsl:434-533).
-__global__ void __launch_bounds__(kQueryThreads) k_scene_query(DeviceWorld w, dyn_query_record* queries,
-                                                               dyn_query_hit_record* hits, uint32_t count) {
+// A selected hit's record.
+__device__ __forceinline__ void write_hit(const DeviceWorld& w, const dyn_query_record& q, uint32_t slot, dyn_query_hit_record* out) {
+    const uint32_t row = w.c_owner[slot];
+    const DBody b = load_dbody(w.hot, row);
+    const QHit hit = resolve_hit(w, q, world_shape(b.position, b.orientation, load_dcoll(w, slot)), true);
+    const uint4 ident = w.ident[row];
+    dyn_query_hit_record r;
+    r.body_id = ident.x;
+    r.body_generation = ident.y;
+    r.distance = hit.distance;
+    r.scene_target = (DYN_ENTRY_KIND_COLLIDER << DYN_ENTRY_KIND_SHIFT) | slot;
+    r.point[0] = hit.point.x;
+    r.point[1] = hit.point.y;
+    r.point[2] = hit.point.z;
+    r.triangle = hit.triangle;
+    r.normal[0] = hit.normal.x;
+    r.normal[1] = hit.normal.y;
+    r.normal[2] = hit.normal.z;
+    r.surface = DYN_NO_SURFACE;  // hull triangles carry no surface (crates/dynamis-world/src/shape_pool.rs:557-580)
+    *out = r;
+}
+
+// Can a ray of this query reach the box at all? Every ray test is analytic, so a ray that clears the
+// box by more than the tests' rounding meets nothing in it. The largest rounding is that of a
+// quadratic's discriminant, about 5e-7 of the squared distance, which answers a miss by up to 7e-4 of
+// the distance as a hit: the box is grown by three times that and a millimetre.
+__device__ __forceinline__ bool ray_meets(f3 origin, f3 heading, float extent, f3 mn, f3 mx) {
+    const f3 far = vmax(vabs(mn - origin), vabs(mx - origin));
+    const float slack = 1e-3f + 2e-3f * (far.x + far.y + far.z);
+    float near_t = -slack, far_t = extent + slack;
+    for (uint32_t axis = 0; axis < 3u; ++axis) {
+        const float o = comp(origin, axis), d = comp(heading, axis);
+        const float lo = comp(mn, axis) - slack, hi = comp(mx, axis) + slack;
+        if (fabsf(d) < 1e-6f) {  // it drifts by less than the slack over its length, or starts outside
+            if ((o < lo || o > hi) && extent < 1e3f) return false;
+            continue;
+        }
+        const float a = (lo - o) / d, b = (hi - o) / d;
+        near_t = fmaxf(near_t, fminf(a, b));
+        far_t = fminf(far_t, fmaxf(a, b));
+    }
+    return !(near_t > far_t + slack);
+}
+
+// A warp's queries keep their candidates in 6 KB of shared memory, so sixteen run on an SM.
+constexpr uint32_t kWarpCandidates = 512u;
+struct QueryWarpShared {
+    unsigned long long keys[kWarpCandidates];
+    uint32_t candidates[kWarpCandidates];
+    uint32_t seen, kept;  // candidates met, and those of them a ray can meet
+};
+// block_bitonic by one warp.
+template <typename T>
+__device__ __forceinline__ void warp_bitonic(T* values, uint32_t width) {
+    const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll 1
+    for (uint32_t k = 2u; k <= width; k <<= 1) {
+#pragma unroll 1
+        for (uint32_t j = k >> 1; j > 0u; j >>= 1) {
+#pragma unroll 1
+            for (uint32_t index = lane; index < width; index += 32u) {
+                const uint32_t other = index ^ j;
+                if (other > index) {
+                    const bool ascending = (index & k) == 0u;
+                    const T a = values[index], b = values[other];
+                    if (ascending ? a > b : a < b) {
+                        values[index] = b;
+                        values[other] = a;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
+// One warp per query (scene_cast.wgsl:434-533), taken from a shared ticket. A block per query left
+// three of its four warps waiting at barriers for the one that tested hits (7 of 16 cycles per
+// instruction), and tested candidates where they lay among their duplicates (8 of 32 threads per
+// instruction): here the distinct ones are packed first, and a ray's candidates that its box test
+// rules out are dropped before the sort. A query with more candidates than the warp holds goes to
+// k_scene_query_large.
+__global__ void __launch_bounds__(kQueryThreads) k_scene_query(DeviceWorld w, dyn_query_record* queries, dyn_query_hit_record* hits,
+                                                               uint32_t count, uint32_t* __restrict__ large) {
+    __shared__ QueryWarpShared shared[kQueryThreads / 32u];
+    QueryWarpShared& sh = shared[threadIdx.x >> 5];
+    const uint32_t lane = threadIdx.x & 31u, lane_lt = (1u << lane) - 1u;
+    const uint32_t live = min(w.ctl[CTL_ENTRIES], w.e_cap);
+    const float grid = base_cell(w);
+    const uint32_t bits = cell_table_bits(w, live);
+    const bool table_overflow = w.ctl[CTL_CELL_OVERFLOW] != 0u;
+    const uint32_t levels = w.counters[DYN_COUNTER_GRID_LEVELS] | w.counters[DYN_COUNTER_RESTING_LEVELS] |
+                            w.counters[DYN_COUNTER_IMMOVABLE_LEVELS];
+    for (;;) {
+        uint32_t qi = 0u;
+        if (lane == 0u) qi = atomicAdd(&w.ctl[CTL_QUERY_NEXT], 1u);
+        qi = __shfl_sync(kFull, qi, 0);
+        if (qi >= count) break;
+        const dyn_query_record q = queries[qi];
+        if (lane == 0u) sh.seen = sh.kept = 0u;
+        __syncwarp();
+        // the candidates: entries of the cells the query's box covers, level by level
+        const DAabb box = query_box(w, q);
+        const bool is_ray = q.kind == DYN_QUERY_RAY;
+        const f3 origin = q_origin(q), heading = is_ray ? normalize(q_direction(q)) : s3(0.0f);
+        auto push = [&](const GEntry& e) {
+            const uint32_t seen = atomicAdd(&sh.seen, 1u);
+            if (seen >= DYN_QUERY_CANDIDATES) return;
+            if (is_ray && !ray_meets(origin, heading, q.extent, e.mn, e.mx)) return;
+            const uint32_t at = atomicAdd(&sh.kept, 1u);
+            if (at < kWarpCandidates) sh.candidates[at] = e.info & DYN_ENTRY_INDEX_MASK;
+        };
+        uint32_t occupied = (q.filters.targets & DYN_QUERY_TARGET_COLLIDERS) != 0u ? levels : 0u;
+#pragma unroll 1
+        while (occupied != 0u) {
+            const uint32_t level = (uint32_t)__ffs(occupied) - 1u;
+            occupied &= occupied - 1u;
+            const float cs = level_size(level, grid);
+            const I3 lo = floor_div(box.min, cs), hi = floor_div(box.max, cs);
+            const long long sx = (long long)hi.x - lo.x + 1, sy = (long long)hi.y - lo.y + 1, sz = (long long)hi.z - lo.z + 1;
+            const long long cells = sx * sy * sz;
+            if (cells <= 0) continue;
+            if (cells > (long long)kGridWalkCells) {
+                // the whole level, its entries tested against the box
+                const uint32_t first = lower_bound(w.ekey, live, level << DYN_LEVEL_KEY_SHIFT);
+                const uint32_t end = lower_bound(w.ekey, live, (level + 1u) << DYN_LEVEL_KEY_SHIFT);
+                for (uint32_t j = first + lane; j < end && sh.seen <= DYN_QUERY_CANDIDATES; j += 32u) {
+                    const GEntry e = load_entry(w, w.eval[j]);
+                    if (!(e.mn.x <= box.max.x && e.mn.y <= box.max.y && e.mn.z <= box.max.z && box.min.x <= e.mx.x &&
+                          box.min.y <= e.mx.y && box.min.z <= e.mx.z))
+                        continue;
+                    push(e);
+                }
+            } else {
+                const uint32_t rows = (uint32_t)(sy * sz);
+                for (uint32_t c = lane; c < (uint32_t)cells; c += 32u) {
+                    const I3 cell = I3{lo.x + (int)(c / rows), lo.y + (int)((c / (uint32_t)sz) % (uint32_t)sy), lo.z + (int)(c % (uint32_t)sz)};
+                    const uint32_t key = cell_key(level, cell);
+                    uint32_t j = cell_find(w, live, bits, table_overflow, key);
+                    if (j >= live) continue;
+                    const uint32_t end = j + __ldg(&w.erun[j].y);
+                    for (; j < end; ++j) push(load_entry(w, w.eval[j]));
+                }
+            }
+        }
+        __syncwarp();
+        const uint32_t total = sh.kept;
+        if (total > kWarpCandidates || sh.seen > DYN_QUERY_CANDIDATES) {
+            if (lane == 0u) large[atomicAdd(&w.ctl[CTL_QUERY_LARGE], 1u)] = qi;
+            __syncwarp();
+            continue;
+        }
+        uint32_t width = 1u;
+        while (width < total) width <<= 1;
+        for (uint32_t i = total + lane; i < width; i += 32u) sh.candidates[i] = 0xFFFFFFFFu;
+        __syncwarp();
+        warp_bitonic(sh.candidates, width);
+        // the distinct ones (a collider has an entry per covered cell) that pass the filters, packed
+        uint32_t distinct = 0u;
+#pragma unroll 1
+        for (uint32_t base = 0; base < total; base += 32u) {
+            const uint32_t i = base + lane;
+            uint32_t slot = 0u;
+            bool keep = false;
+            if (i < total) {
+                slot = sh.candidates[i];
+                keep = (i == 0u || sh.candidates[i - 1u] != slot) && query_passes(w, q, slot);
+            }
+            const uint32_t mask = __ballot_sync(kFull, keep);
+            // the words written lie before the ones later rounds read, except the last word of this
+            // round, which the next compares with: the packed slots go to the keys' space
+            if (keep) reinterpret_cast<uint32_t*>(sh.keys)[kWarpCandidates + distinct + __popc(mask & lane_lt)] = slot;
+            distinct += __popc(mask);
+        }
+        __syncwarp();
+        for (uint32_t i = lane; i < distinct; i += 32u) sh.candidates[i] = reinterpret_cast<const uint32_t*>(sh.keys)[kWarpCandidates + i];
+        __syncwarp();
+        // their hits, keyed by (distance key, candidate)
+        uint32_t hit_total = 0u;
+#pragma unroll 1
+        for (uint32_t base = 0; base < distinct; base += 32u) {
+            const uint32_t i = base + lane;
+            unsigned long long key = 0ull;
+            bool found = false;
+            if (i < distinct) {
+                const uint32_t slot = sh.candidates[i];
+                const DBody b = load_dbody(w.hot, w.c_owner[slot]);
+                const QHit hit = resolve_hit(w, q, world_shape(b.position, b.orientation, load_dcoll(w, slot)), false);
+                found = hit.distance < kQNoHit;
+                key = ((unsigned long long)hit_key(hit.distance) << 32) | slot;
+            }
+            const uint32_t mask = __ballot_sync(kFull, found);
+            if (found) sh.keys[hit_total + __popc(mask & lane_lt)] = key;
+            hit_total += __popc(mask);
+        }
+        uint32_t sorted = 1u;
+        while (sorted < hit_total) sorted <<= 1;
+        for (uint32_t i = hit_total + lane; i < sorted; i += 32u) sh.keys[i] = ~0ull;
+        __syncwarp();
+        warp_bitonic(sh.keys, sorted);
+        const uint32_t emitted = min(min(q.max_hits, DYN_QUERY_CANDIDATES), hit_total);
+#pragma unroll 1
+        for (uint32_t i = lane; i < emitted; i += 32u) write_hit(w, q, (uint32_t)(sh.keys[i] & 0xFFFFFFFFull), hits + q.hit_base + i);
+        if (lane == 0u) {
+            queries[qi].count = emitted;
+            queries[qi].overflow = emitted < hit_total ? 1u : 0u;
+        }
+        __syncwarp();
+    }
+}
+
+// One block per query (scene_cast.wgsl:434-533), for the queries with more candidates than a warp holds.
+__global__ void __launch_bounds__(kQueryThreads) k_scene_query_large(DeviceWorld w, dyn_query_record* queries,
+                                                                     dyn_query_hit_record* hits, const uint32_t* __restrict__ list) {
     extern __shared__ __align__(16) unsigned char smem[];
     QueryShared& sh = *reinterpret_cast<QueryShared*>(smem);
-    for (uint32_t qi = blockIdx.x; qi < count; qi += gridDim.x) {
+    const uint32_t count = w.ctl[CTL_QUERY_LARGE];
+    for (uint32_t at = blockIdx.x; at < count; at += gridDim.x) {
+        const uint32_t qi = list[at];
         const dyn_query_record q = queries[qi];
         if (threadIdx.x == 0) {
             sh.candidate_count = 0u;
@@ -604,7 +822,7 @@ __global__ void __launch_bounds__(kQueryThreads) k_scene_query(DeviceWorld w, dy
                 if (query_passes(w, q, slot)) {
                     const uint32_t row = w.c_owner[slot];
                     const DBody b = load_dbody(w.hot, row);
-                    const QHit hit = resolve_hit(w, q, world_shape(b.position, b.orientation, load_dcoll(w, slot)));
+                    const QHit hit = resolve_hit(w, q, world_shape(b.position, b.orientation, load_dcoll(w, slot)), false);
                     if (hit.distance < kQNoHit) {
                         key = ((unsigned long long)hit_key(hit.distance) << 32) | slot;
                         atomicAdd(&sh.hit_total, 1u);
@@ -615,28 +833,9 @@ __global__ void __launch_bounds__(kQueryThreads) k_scene_query(DeviceWorld w, dy
         }
         __syncthreads();
         block_bitonic(sh.keys, width);
-        const uint32_t capacity = min(q.max_hits, DYN_QUERY_CANDIDATES);
-        const uint32_t emitted = min(capacity, sh.hit_total);
+        const uint32_t emitted = min(min(q.max_hits, DYN_QUERY_CANDIDATES), sh.hit_total);
         for (uint32_t i = threadIdx.x; i < emitted; i += blockDim.x) {
-            const uint32_t slot = (uint32_t)(sh.keys[i] & 0xFFFFFFFFull);
-            const uint32_t row = w.c_owner[slot];
-            const DBody b = load_dbody(w.hot, row);
-            const QHit hit = resolve_hit(w, q, world_shape(b.position, b.orientation, load_dcoll(w, slot)));
-            const uint4 ident = w.ident[row];
-            dyn_query_hit_record r;
-            r.body_id = ident.x;
-            r.body_generation = ident.y;
-            r.distance = hit.distance;
-            r.scene_target = (DYN_ENTRY_KIND_COLLIDER << DYN_ENTRY_KIND_SHIFT) | slot;
-            r.point[0] = hit.point.x;
-            r.point[1] = hit.point.y;
-            r.point[2] = hit.point.z;
-            r.triangle = hit.triangle;
-            r.normal[0] = hit.normal.x;
-            r.normal[1] = hit.normal.y;
-            r.normal[2] = hit.normal.z;
-            r.surface = DYN_NO_SURFACE;  // hull triangles carry no surface (crates/dynamis-world/src/shape_pool.rs:557-580)
-            hits[q.hit_base + i] = r;
+            write_hit(w, q, (uint32_t)(sh.keys[i] & 0xFFFFFFFFull), hits + q.hit_base + i);
         }
         if (threadIdx.x == 0) {
             queries[qi].count = emitted;

@@ -109,6 +109,7 @@ struct DeviceState {
     // a query batch's records and hits on the device (dyn_query), grown as batches need
     dyn_query_record* query_buf = nullptr;
     dyn_query_hit_record* hit_buf = nullptr;
+    uint32_t* query_list = nullptr;  // [query_cap] the batch's queries with many candidates
     // a query's own grid: its entries and its counters and control words, so that a query between
     // steps leaves the step's kept grid runs and counters as they were
     float4* query_entries = nullptr;
@@ -1143,6 +1144,7 @@ void destroy_device(dyn_world* w) {
     if (d->edit_buffer) cudaFree(d->edit_buffer);
     if (d->edit_run_buffer) cudaFree(d->edit_run_buffer);
     if (d->query_buf) cudaFree(d->query_buf);
+    if (d->query_list) cudaFree(d->query_list);
     if (d->hit_buf) cudaFree(d->hit_buf);
     if (d->query_entries) cudaFree(d->query_entries);
     if (d->query_words) cudaFree(d->query_words);
@@ -2397,8 +2399,12 @@ DYN_API dyn_status dyn_query(dyn_world* w, dyn_query_record* queries, uint32_t n
     if (n > d->query_cap) {
         DYN_CUDA(cudaStreamSynchronize(d->stream));
         if (d->query_buf) cudaFree(d->query_buf);
+        if (d->query_list) cudaFree(d->query_list);
         d->query_buf = nullptr;
+        d->query_list = nullptr;
+        d->query_cap = 0;
         DYN_CUDA(cudaMalloc(&d->query_buf, (size_t)n * sizeof(dyn_query_record)));
+        DYN_CUDA(cudaMalloc(&d->query_list, (size_t)n * sizeof(uint32_t)));
         d->query_cap = n;
     }
     if (base > d->hit_cap) {
@@ -2437,8 +2443,10 @@ DYN_API dyn_status dyn_query(dyn_world* w, dyn_query_record* queries, uint32_t n
     k_cell_insert<<<blocks_for(d, E, 256), 256, 0, s>>>(dw);
     DYN_CUDA(cudaMemcpyAsync(d->query_buf, queries, (size_t)n * sizeof(dyn_query_record), cudaMemcpyHostToDevice, s));
     const size_t smem = sizeof(QueryShared);
-    DYN_CUDA(cudaFuncSetAttribute(k_scene_query, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_scene_query<<<std::min<uint32_t>(n, d->sms * 4u), kQueryThreads, smem, s>>>(dw, d->query_buf, d->hit_buf, n);
+    DYN_CUDA(cudaFuncSetAttribute(k_scene_query_large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_scene_query<<<std::min<uint32_t>(div_up(n, kQueryThreads / 32u), d->sms * 4u), kQueryThreads, 0, s>>>(dw, d->query_buf, d->hit_buf,
+                                                                                                  n, d->query_list);
+    k_scene_query_large<<<std::min<uint32_t>(n, d->sms * 4u), kQueryThreads, smem, s>>>(dw, d->query_buf, d->hit_buf, d->query_list);
     DYN_CUDA(cudaGetLastError());
     DYN_CUDA(cudaMemcpyAsync(queries, d->query_buf, (size_t)n * sizeof(dyn_query_record), cudaMemcpyDeviceToHost, s));
     if (base) DYN_CUDA(cudaMemcpyAsync(hits, d->hit_buf, (size_t)base * sizeof(dyn_query_hit_record), cudaMemcpyDeviceToHost, s));
