@@ -305,13 +305,6 @@ __device__ __forceinline__ f3 q_direction(const dyn_query_record& q) {
     return mk3(q.direction[0], q.direction[1], q.direction[2]);
 }
 
-// convex.wgsl:627-630: convex_hit with the normal turned to face the probe
-__device__ __forceinline__ Hit penetration_hit(const DeviceWorld& w, const WShape& probe, const WShape& solid) {
-    Hit h = convex_hit(w, probe, solid);
-    h.normal = -h.normal;
-    return h;
-}
-
 // scene.wgsl:536-555 for one hull triangle in the hull's frame
 struct QClosest {
     float distance;
@@ -368,23 +361,6 @@ __device__ float overlap_world_geom(const DeviceWorld& w, const dyn_query_record
     return distance;
 }
 
-// overlap_hit (scene_cast.wgsl:160-178)
-__device__ float overlap_hit(const DeviceWorld& w, const dyn_query_record& q, const WShape& world, f3* out_normal) {
-    WShape probe = query_probe(q, q_origin(q));
-    probe.radius = 0.0f;
-    const GjkOut closest = gjk_phase(w, probe, world);
-    if (closest.pen) {
-        const Hit hit = penetration_hit(w, query_probe(q, q_origin(q)), world);
-        *out_normal = hit.normal;
-        return -q.extent + wmax(hit.distance + q.extent, 0.0f);
-    }
-    if (closest.dist <= q.extent) {
-        *out_normal = -closest.normal;
-        return closest.dist - q.extent;
-    }
-    return kQNoHit;
-}
-
 // shape_sweep (scene.wgsl:219-257) of the query's shape against a collider
 __device__ QHit shape_sweep(const DeviceWorld& w, const WShape& moving, const WShape& target, f3 start, f3 direction,
                             float max_dist) {
@@ -413,46 +389,72 @@ __device__ QHit shape_sweep(const DeviceWorld& w, const WShape& moving, const WS
     return q_no_hit();
 }
 
-// resolve_hit (scene_cast.wgsl:384-432) of one collider. Without `whole` only the distance is wanted
-// (the selection's first pass over the candidates): a sphere or point query then leaves out the walk
-// over a hull's triangles that gives its normal, which a miss never needs either.
-__device__ QHit resolve_hit(const DeviceWorld& w, const dyn_query_record& q, const WShape& world, bool whole) {
+// resolve_hit (scene_cast.wgsl:384-432) of one collider, as far as one lane takes it: a probe that its
+// closest-point search finds inside the collider (`inside`) has its depth and normal from finish_inside.
+// Without `whole` only the distance is wanted (the selection's first pass over the candidates): a
+// sphere or point query then leaves out the walk over a hull's triangles that gives its normal, which
+// a miss never needs either.
+struct Resolved {
+    QHit hit;
+    bool inside;
+};
+__device__ __forceinline__ void geom_normal(const DeviceWorld& w, const dyn_query_record& q, const WShape& world, QHit* hit) {
+    f3 normal = hit->normal;
+    overlap_world_geom(w, q, world, &normal);
+    hit->normal = normal;
+}
+__device__ Resolved resolve_lane(const DeviceWorld& w, const dyn_query_record& q, const WShape& world, bool whole) {
     const uint32_t kind = q.kind;
     if (kind == DYN_QUERY_RAY) {
         const f3 direction = normalize(q_direction(q));
         QHit hit = shape_ray(w, world, q_origin(q), direction, q.extent);
-        if (hit.distance == kQNoHit) return hit;
+        if (hit.distance == kQNoHit) return Resolved{hit, false};
         if (dot(hit.normal, direction) > 0.0f) hit.normal = -hit.normal;
-        return hit;
+        return Resolved{hit, false};
     }
-    const bool world_geom = shape_world_geometry(world.kind);
     if (kind == DYN_QUERY_SWEEP) {
         const QHit hit = shape_sweep(w, query_probe(q, q_origin(q)), world, q_origin(q), q_direction(q), q.extent);
-        return hit.distance < kQNoHit ? hit : q_no_hit();
+        return Resolved{hit.distance < kQNoHit ? hit : q_no_hit(), false};
     }
-    f3 normal = s3(0.0f);
-    if (kind == DYN_QUERY_SPHERE || kind == DYN_QUERY_POINT) {
-        float separation = world_geom ? 0.0f : overlap_hit(w, q, world, &normal);
-        if (world_geom) {
-            separation = overlap_world_geom(w, q, world, &normal);
-        } else if (whole && separation < kQNoHit) {
-            overlap_world_geom(w, q, world, &normal);
-        }
-        if (separation < kQNoHit) return QHit{separation, world.center, normal, DYN_NO_TRIANGLE};
-        return q_no_hit();
-    }
-    if (world_geom) {
+    if (shape_world_geometry(world.kind)) {
+        f3 normal = s3(0.0f);
         const float separation = overlap_world_geom(w, q, world, &normal);
-        if (separation < kQNoHit) return QHit{separation, world.center, normal, DYN_NO_TRIANGLE};
-        return q_no_hit();
+        if (separation < kQNoHit) return Resolved{QHit{separation, world.center, normal, DYN_NO_TRIANGLE}, false};
+        return Resolved{q_no_hit(), false};
     }
-    const WShape probe = query_probe(q, q_origin(q));
+    const bool ball = kind == DYN_QUERY_SPHERE || kind == DYN_QUERY_POINT;
+    WShape probe = query_probe(q, q_origin(q));
+    if (ball) probe.radius = 0.0f;  // overlap_hit (scene_cast.wgsl:160-178)
     const GjkOut closest = gjk_phase(w, probe, world);
-    if (closest.pen) {
-        const Hit hit = penetration_hit(w, probe, world);
-        return QHit{hit.distance, (closest.pa + closest.pb) * 0.5f, hit.normal, DYN_NO_TRIANGLE};
+    if (!ball) {
+        if (!closest.pen) return Resolved{q_no_hit(), false};
+        return Resolved{QHit{0.0f, (closest.pa + closest.pb) * 0.5f, s3(0.0f), DYN_NO_TRIANGLE}, true};
     }
-    return q_no_hit();
+    if (closest.pen) return Resolved{QHit{0.0f, world.center, s3(0.0f), DYN_NO_TRIANGLE}, true};
+    if (!(closest.dist <= q.extent)) return Resolved{q_no_hit(), false};
+    QHit hit{closest.dist - q.extent, world.center, -closest.normal, DYN_NO_TRIANGLE};
+    if (!(hit.distance < kQNoHit)) return Resolved{q_no_hit(), false};
+    if (whole) geom_normal(w, q, world, &hit);
+    return Resolved{hit, false};
+}
+// The rest of an inside probe's hit from the penetration `h` of query_probe in the collider
+// (convex_hit with the normal turned to face the probe, convex.wgsl:627-630).
+__device__ __forceinline__ void finish_inside(const DeviceWorld& w, const dyn_query_record& q, const WShape& world, const Hit& h,
+                                              bool whole, QHit* hit) {
+    hit->normal = -h.normal;
+    hit->distance = h.distance;
+    if (q.kind != DYN_QUERY_SPHERE && q.kind != DYN_QUERY_POINT) return;
+    hit->distance = -q.extent + wmax(h.distance + q.extent, 0.0f);
+    if (!(hit->distance < kQNoHit)) {
+        *hit = q_no_hit();
+    } else if (whole) {
+        geom_normal(w, q, world, hit);
+    }
+}
+__device__ QHit resolve_hit(const DeviceWorld& w, const dyn_query_record& q, const WShape& world, bool whole) {
+    Resolved r = resolve_lane(w, q, world, whole);
+    if (r.inside) finish_inside(w, q, world, convex_hit(w, query_probe(q, q_origin(q)), world), whole, &r.hit);
+    return r.hit;
 }
 
 // body_passes (scene_cast.wgsl:196-222) and collider_filter_query (core.wgsl:285-291)
@@ -538,12 +540,13 @@ __device__ __forceinline__ void push_candidate(QueryShared& sh, uint32_t slot) {
     sh.candidates[at] = slot;
 }
 
+__device__ __forceinline__ WShape collider_shape(const DeviceWorld& w, uint32_t slot) {
+    const DBody b = load_dbody(w.hot, w.c_owner[slot]);
+    return world_shape(b.position, b.orientation, load_dcoll(w, slot));
+}
 // A selected hit's record.
-__device__ __forceinline__ void write_hit(const DeviceWorld& w, const dyn_query_record& q, uint32_t slot, dyn_query_hit_record* out) {
-    const uint32_t row = w.c_owner[slot];
-    const DBody b = load_dbody(w.hot, row);
-    const QHit hit = resolve_hit(w, q, world_shape(b.position, b.orientation, load_dcoll(w, slot)), true);
-    const uint4 ident = w.ident[row];
+__device__ __forceinline__ void write_hit(const DeviceWorld& w, const QHit& hit, uint32_t slot, dyn_query_hit_record* out) {
+    const uint4 ident = w.ident[w.c_owner[slot]];
     dyn_query_hit_record r;
     r.body_id = ident.x;
     r.body_generation = ident.y;
@@ -582,9 +585,12 @@ __device__ __forceinline__ bool ray_meets(f3 origin, f3 heading, float extent, f
     return !(near_t > far_t + slack);
 }
 
-// A warp's queries keep their candidates in 6 KB of shared memory, so sixteen run on an SM.
+// A warp's queries keep their candidates in 6 KB of shared memory and a polytope in 4, so sixteen run
+// on an SM.
 constexpr uint32_t kWarpCandidates = 512u;
 struct QueryWarpShared {
+    EpaWarpShared epa;
+    SPt simplex[4];
     unsigned long long keys[kWarpCandidates];
     uint32_t candidates[kWarpCandidates];
     uint32_t seen, kept;  // candidates met, and those of them a ray can meet
@@ -614,6 +620,28 @@ __device__ __forceinline__ void warp_bitonic(T* values, uint32_t width) {
     }
 }
 
+// resolve_hit for a slot per lane (has: this lane holds one). The lanes search for their own closest
+// points; then the whole warp takes the inside probes' penetrations in turn (group_convex_hit), which on
+// one lane, the polytope in its local memory, were most of a sphere query's time.
+__device__ __forceinline__ QHit warp_resolve(const Lanes<32>& L, const DeviceWorld& w, const dyn_query_record& q, bool has, uint32_t slot,
+                                             bool whole, QueryWarpShared& sh) {
+    Resolved r{q_no_hit(), false};
+    if (has) r = resolve_lane(w, q, collider_shape(w, slot), whole);
+    uint32_t inside = __ballot_sync(kFull, r.inside);
+    if (inside == 0u) return r.hit;
+    const GroupShape<32> probe = group_shape(L, w, query_probe(q, q_origin(q)));
+#pragma unroll 1
+    while (inside != 0u) {
+        const uint32_t from = (uint32_t)__ffs(inside) - 1u;
+        inside &= inside - 1u;
+        const WShape solid = collider_shape(w, L.shfl(slot, from));
+        const Hit h = group_convex_hit(L, w, probe, group_shape(L, w, solid), sh.simplex, sh.epa);
+        if (L.lane == from) finish_inside(w, q, solid, h, whole, &r.hit);
+        __syncwarp();
+    }
+    return r.hit;
+}
+
 // One warp per query (scene_cast.wgsl:434-533), taken from a shared ticket. A block per query left
 // three of its four warps waiting at barriers for the one that tested hits (7 of 16 cycles per
 // instruction), and tested candidates where they lay among their duplicates (8 of 32 threads per
@@ -624,7 +652,8 @@ __global__ void __launch_bounds__(kQueryThreads) k_scene_query(DeviceWorld w, dy
                                                                uint32_t count, uint32_t* __restrict__ large) {
     __shared__ QueryWarpShared shared[kQueryThreads / 32u];
     QueryWarpShared& sh = shared[threadIdx.x >> 5];
-    const uint32_t lane = threadIdx.x & 31u, lane_lt = (1u << lane) - 1u;
+    const Lanes<32> L;
+    const uint32_t lane = L.lane, lane_lt = (1u << lane) - 1u;
     const uint32_t live = min(w.ctl[CTL_ENTRIES], w.e_cap);
     const float grid = base_cell(w);
     const uint32_t bits = cell_table_bits(w, live);
@@ -720,15 +749,11 @@ __global__ void __launch_bounds__(kQueryThreads) k_scene_query(DeviceWorld w, dy
 #pragma unroll 1
         for (uint32_t base = 0; base < distinct; base += 32u) {
             const uint32_t i = base + lane;
-            unsigned long long key = 0ull;
-            bool found = false;
-            if (i < distinct) {
-                const uint32_t slot = sh.candidates[i];
-                const DBody b = load_dbody(w.hot, w.c_owner[slot]);
-                const QHit hit = resolve_hit(w, q, world_shape(b.position, b.orientation, load_dcoll(w, slot)), false);
-                found = hit.distance < kQNoHit;
-                key = ((unsigned long long)hit_key(hit.distance) << 32) | slot;
-            }
+            const bool has = i < distinct;
+            const uint32_t slot = has ? sh.candidates[i] : 0u;
+            const QHit hit = warp_resolve(L, w, q, has, slot, false, sh);
+            const bool found = hit.distance < kQNoHit;
+            const unsigned long long key = ((unsigned long long)hit_key(hit.distance) << 32) | slot;
             const uint32_t mask = __ballot_sync(kFull, found);
             if (found) sh.keys[hit_total + __popc(mask & lane_lt)] = key;
             hit_total += __popc(mask);
@@ -740,7 +765,13 @@ __global__ void __launch_bounds__(kQueryThreads) k_scene_query(DeviceWorld w, dy
         warp_bitonic(sh.keys, sorted);
         const uint32_t emitted = min(min(q.max_hits, DYN_QUERY_CANDIDATES), hit_total);
 #pragma unroll 1
-        for (uint32_t i = lane; i < emitted; i += 32u) write_hit(w, q, (uint32_t)(sh.keys[i] & 0xFFFFFFFFull), hits + q.hit_base + i);
+        for (uint32_t base = 0; base < emitted; base += 32u) {
+            const uint32_t i = base + lane;
+            const bool has = i < emitted;
+            const uint32_t slot = has ? (uint32_t)(sh.keys[i] & 0xFFFFFFFFull) : 0u;
+            const QHit hit = warp_resolve(L, w, q, has, slot, true, sh);
+            if (has) write_hit(w, hit, slot, hits + q.hit_base + i);
+        }
         if (lane == 0u) {
             queries[qi].count = emitted;
             queries[qi].overflow = emitted < hit_total ? 1u : 0u;
@@ -820,9 +851,7 @@ __global__ void __launch_bounds__(kQueryThreads) k_scene_query_large(DeviceWorld
             if (i < total && !(i > 0u && sh.candidates[i] == sh.candidates[i - 1u])) {
                 const uint32_t slot = sh.candidates[i];
                 if (query_passes(w, q, slot)) {
-                    const uint32_t row = w.c_owner[slot];
-                    const DBody b = load_dbody(w.hot, row);
-                    const QHit hit = resolve_hit(w, q, world_shape(b.position, b.orientation, load_dcoll(w, slot)), false);
+                    const QHit hit = resolve_hit(w, q, collider_shape(w, slot), false);
                     if (hit.distance < kQNoHit) {
                         key = ((unsigned long long)hit_key(hit.distance) << 32) | slot;
                         atomicAdd(&sh.hit_total, 1u);
@@ -835,7 +864,8 @@ __global__ void __launch_bounds__(kQueryThreads) k_scene_query_large(DeviceWorld
         block_bitonic(sh.keys, width);
         const uint32_t emitted = min(min(q.max_hits, DYN_QUERY_CANDIDATES), sh.hit_total);
         for (uint32_t i = threadIdx.x; i < emitted; i += blockDim.x) {
-            write_hit(w, q, (uint32_t)(sh.keys[i] & 0xFFFFFFFFull), hits + q.hit_base + i);
+            const uint32_t slot = (uint32_t)(sh.keys[i] & 0xFFFFFFFFull);
+            write_hit(w, resolve_hit(w, q, collider_shape(w, slot), true), slot, hits + q.hit_base + i);
         }
         if (threadIdx.x == 0) {
             queries[qi].count = emitted;
