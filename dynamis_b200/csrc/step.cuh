@@ -552,20 +552,50 @@ __device__ __forceinline__ bool same_cell(I3 a, I3 b) { return a.x == b.x && a.y
 __device__ __forceinline__ bool overlap_cell_is(const GEntry& a, const GEntry& b, float cs, I3 cell) {
     return same_cell(floor_div(vmax(a.mn, b.mn), cs), cell);
 }
-__device__ __forceinline__ void emit_pair(const DeviceWorld& w, const GEntry& a, const GEntry& b, bool same_node) {
+// Emitted pairs gather in shared memory and leave a block at a time: one atomic on the pair counter for
+// hundreds of pairs, and coalesced stores. With an atomic for every few lanes that emit together, the
+// counter's one address was what k_pairs_coarse and k_pairs_cell waited for on large worlds.
+constexpr uint32_t kPairStage = 1024u;
+struct PairStage {
+    uint32_t count, base;
+    uint2 pairs[kPairStage];
+};
+__device__ __forceinline__ void store_pair(const DeviceWorld& w, uint32_t slot, uint2 pair) {
+    if (slot < w.p_cap) {
+        w.pmaj[slot] = pair.x;
+        w.pmin[slot] = pair.y;
+    } else {
+        add_counter(&w.counters[DYN_COUNTER_REFUSED_PAIRS], 1u);
+    }
+}
+__device__ __forceinline__ void emit_pair(const DeviceWorld& w, PairStage& stage, const GEntry& a, const GEntry& b, bool same_node) {
     if (((a.info & DYN_ENTRY_KIND_MASK) >> DYN_ENTRY_KIND_SHIFT) != DYN_ENTRY_KIND_COLLIDER) return;
     if (((b.info & DYN_ENTRY_KIND_MASK) >> DYN_ENTRY_KIND_SHIFT) != DYN_ENTRY_KIND_COLLIDER) return;
     if (same_node || a.group == b.group) return;
     if ((a.info & DYN_ENTRY_MOBILE) == 0u && (b.info & DYN_ENTRY_MOBILE) == 0u) return;
     if (w.body_world[a.group] != w.body_world[b.group]) return;  // different sub-worlds of a batch
-    uint32_t slot = append_slot(&w.counters[DYN_COUNTER_PAIRS]);
-    if (slot < w.p_cap) {
-        uint32_t ia = a.info & DYN_ENTRY_INDEX_MASK, ib = b.info & DYN_ENTRY_INDEX_MASK;
-        w.pmaj[slot] = min(ia, ib);
-        w.pmin[slot] = max(ia, ib);
-    } else {
-        add_counter(&w.counters[DYN_COUNTER_REFUSED_PAIRS], 1u);
+    const uint32_t ia = a.info & DYN_ENTRY_INDEX_MASK, ib = b.info & DYN_ENTRY_INDEX_MASK;
+    const uint2 pair = make_uint2(min(ia, ib), max(ia, ib));
+    const uint32_t at = append_slot(&stage.count);
+    if (at < kPairStage) {
+        stage.pairs[at] = pair;
+    } else {  // the block emitted more than it can hold before its next flush
+        store_pair(w, append_slot(&w.counters[DYN_COUNTER_PAIRS]), pair);
     }
+}
+// The block's staged pairs into the stream once there are `enough`. Every thread of the block calls it.
+__device__ __forceinline__ void flush_pairs(const DeviceWorld& w, PairStage& stage, uint32_t enough) {
+    __syncthreads();
+    const uint32_t n = min(stage.count, kPairStage);
+    __syncthreads();  // every thread has read the count before any goes on to emit again
+    if (n < enough) return;
+    if (threadIdx.x == 0) stage.base = atomicAdd(&w.counters[DYN_COUNTER_PAIRS], n);
+    __syncthreads();
+    const uint32_t base = stage.base;
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) store_pair(w, base + i, stage.pairs[i]);
+    __syncthreads();
+    if (threadIdx.x == 0) stage.count = 0u;
+    __syncthreads();
 }
 __device__ __forceinline__ uint32_t lower_bound(const uint32_t* keys, uint32_t n, uint32_t key) {
     uint32_t lo = 0, hi = n;
@@ -670,14 +700,17 @@ __global__ void __launch_bounds__(128) k_pairs_coarse(DeviceWorld w) {
     const bool coarse_active = w.counters[DYN_COUNTER_COARSE_ACTIVE] != 0u;
     const uint32_t bits = cell_table_bits(w, live);
     const bool overflow = w.ctl[CTL_CELL_OVERFLOW] != 0u;
-    GRID_STRIDE(i, w.k) {
-        if (w.c_run[i] == RUN_NONE) continue;
+    __shared__ PairStage stage;
+    if (threadIdx.x == 0) stage.count = 0u;
+    __syncthreads();
+    auto walk = [&](uint32_t i) {
+        if (w.c_run[i] == RUN_NONE) return;
         const uint32_t node = 8u * i;  // the first of the collider's slots: its primary entry
         GEntry e = load_entry(w, node);
-        if (((e.info & DYN_ENTRY_KIND_MASK) >> DYN_ENTRY_KIND_SHIFT) != DYN_ENTRY_KIND_COLLIDER) continue;
-        if ((e.info & DYN_ENTRY_PRIMARY) == 0u) continue;
+        if (((e.info & DYN_ENTRY_KIND_MASK) >> DYN_ENTRY_KIND_SHIFT) != DYN_ENTRY_KIND_COLLIDER) return;
+        if ((e.info & DYN_ENTRY_PRIMARY) == 0u) return;
         const bool awake = entry_awake(w, e);
-        if (!(awake || coarse_active)) continue;
+        if (!(awake || coarse_active)) return;
         const uint32_t level = w.c_level[e.info & DYN_ENTRY_INDEX_MASK];
         const uint32_t world = w.body_world[e.group];
         const uint32_t coarser = occupied & ~((1u << min(level + 1u, 31u)) - 1u);
@@ -729,26 +762,34 @@ __global__ void __launch_bounds__(128) k_pairs_coarse(DeviceWorld w) {
                                 if (!overlaps(e, o[u])) continue;
                                 if (!same_cell(entry_cell(o[u], cs), cell)) continue;
                                 if (!overlap_cell_is(e, o[u], cs, cell)) continue;
-                                emit_pair(w, e, o[u], false);
+                                emit_pair(w, stage, e, o[u], false);
                             }
                         }
                     }
         }
+    };
+    for (uint32_t base = blockIdx.x * blockDim.x; base < w.k; base += gridDim.x * blockDim.x) {
+        if (base + threadIdx.x < w.k) walk(base + threadIdx.x);
+        flush_pairs(w, stage, kPairStage / 2u);
     }
+    flush_pairs(w, stage, 1u);
 }
 
 // One thread per entry that can start a pair (an awake entry, or an immovable one, whose owner's
 // wake flag makes it awake): a resting entry is never awake, so it only answers.
-__global__ void k_pairs_cell(DeviceWorld w) {
+__global__ void __launch_bounds__(256) k_pairs_cell(DeviceWorld w) {
     const uint32_t live = min(w.ctl[CTL_ENTRIES], w.e_cap);
     const uint32_t starts = min(w.held[HELD_AWAKE] + w.held[HELD_IMMOVABLE], live);
     const float grid = base_cell(w);
-    GRID_STRIDE(t, starts) {
+    __shared__ PairStage stage;
+    if (threadIdx.x == 0) stage.count = 0u;
+    __syncthreads();
+    auto scan = [&](uint32_t t) {
         const uint32_t index = __ldg(w.init_pos + t);
         uint32_t node = w.eval[index];
         GEntry e = load_entry(w, node);
-        if (((e.info & DYN_ENTRY_KIND_MASK) >> DYN_ENTRY_KIND_SHIFT) != DYN_ENTRY_KIND_COLLIDER) continue;
-        if (!entry_awake(w, e)) continue;
+        if (((e.info & DYN_ENTRY_KIND_MASK) >> DYN_ENTRY_KIND_SHIFT) != DYN_ENTRY_KIND_COLLIDER) return;
+        if (!entry_awake(w, e)) return;
         uint32_t level = w.c_level[e.info & DYN_ENTRY_INDEX_MASK];
         float cs = level_size(level, grid);
         I3 cell = entry_cell(e, cs);
@@ -770,10 +811,15 @@ __global__ void k_pairs_cell(DeviceWorld w) {
                 if (!overlaps(e, o[u])) continue;
                 if (!same_cell(entry_cell(o[u], cs), cell)) continue;
                 if (!overlap_cell_is(e, o[u], cs, cell)) continue;
-                emit_pair(w, e, o[u], node == others[u]);
+                emit_pair(w, stage, e, o[u], node == others[u]);
             }
         }
+    };
+    for (uint32_t base = blockIdx.x * blockDim.x; base < starts; base += gridDim.x * blockDim.x) {
+        if (base + threadIdx.x < starts) scan(base + threadIdx.x);
+        flush_pairs(w, stage, kPairStage / 2u);
     }
+    flush_pairs(w, stage, 1u);
 }
 
 // ---- narrowphase (narrowphase.wgsl:518-685) into the staging set, then ordered compaction ----
@@ -837,10 +883,18 @@ __device__ __forceinline__ bool joined_by_joint(const DeviceWorld& w, uint32_t r
     return false;
 }
 
-__global__ void k_pair_class(DeviceWorld w) {
+// The lists' places are taken a block at a time (one atomic per list and 256 pairs): an atomic per warp
+// and list on three addresses took 208 us for 2M pairs.
+constexpr uint32_t kClassThreads = 256u;
+__global__ void __launch_bounds__(kClassThreads) k_pair_class(DeviceWorld w) {
+    __shared__ uint32_t warp_count[PC_COUNT][kClassThreads / 32u], list_base[PC_COUNT];
     const uint32_t pairs = min(w.counters[DYN_COUNTER_PAIRS], w.p_cap);
-    GRID_STRIDE(index, pairs) {
-        const uint4 f = w.c_class[w.pmaj[index]], s = w.c_class[w.pmin[index]];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    for (uint32_t base = blockIdx.x * kClassThreads; base < pairs; base += gridDim.x * kClassThreads) {
+        const uint32_t index = base + threadIdx.x;
+        const bool live = index < pairs;
+        const uint4 none = make_uint4(DYN_NO_BODY, 0u, 0u, 0u);
+        const uint4 f = live ? w.c_class[w.pmaj[index]] : none, s = live ? w.c_class[w.pmin[index]] : none;
         const uint32_t fr = f.x, sr = s.x, fk = f.w & 0xffu, sk = s.w & 0xffu;
         int cls = -1;
         do {
@@ -865,15 +919,27 @@ __global__ void k_pair_class(DeviceWorld w) {
                 cls = PC_ANALYTIC;
             }
         } while (false);
-        if (cls < 0) {
-            continue;  // answered here: no contact
-        } else if (cls == PC_ANALYTIC) {  // one branch per list: an aggregated append needs one target
-            w.np_list[append_slot(&w.ctl[CTL_LIST0 + PC_ANALYTIC])] = index;
-        } else if (cls == PC_BOXES) {
-            w.np_list[(size_t)PC_BOXES * w.p_cap + append_slot(&w.ctl[CTL_LIST0 + PC_BOXES])] = index;
-        } else {
-            w.np_list[(size_t)PC_CONVEX * w.p_cap + append_slot(&w.ctl[CTL_LIST0 + PC_CONVEX])] = index;
+        uint32_t before = 0u;
+#pragma unroll
+        for (int c = 0; c < (int)PC_COUNT; ++c) {
+            const uint32_t mask = __ballot_sync(0xFFFFFFFFu, cls == c);
+            if (cls == c) before = __popc(mask & ((1u << lane) - 1u));
+            if (lane == 0u) warp_count[c][warp] = __popc(mask);
         }
+        __syncthreads();
+        if (threadIdx.x < PC_COUNT) {
+            uint32_t total = 0u;
+            for (uint32_t v = 0; v < kClassThreads / 32u; ++v) {
+                const uint32_t n = warp_count[threadIdx.x][v];
+                warp_count[threadIdx.x][v] = total;
+                total += n;
+            }
+            list_base[threadIdx.x] = total ? atomicAdd(&w.ctl[CTL_LIST0 + threadIdx.x], total) : 0u;
+        }
+        __syncthreads();
+        // a pair that fails a filter is answered here: no contact
+        if (cls >= 0) w.np_list[(size_t)cls * w.p_cap + list_base[cls] + warp_count[cls][warp] + before] = index;
+        __syncthreads();
     }
 }
 

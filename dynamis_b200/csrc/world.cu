@@ -796,7 +796,7 @@ void record_step(dyn_world* w, cudaStream_t s, uint32_t parity, bool timed, cons
     join(0, side);
     // the candidate pairs stay in emission order; the contacts are sorted into pair order below
     mark(ST_NARROWPHASE);
-    k_pair_class<<<blocks_for(d, P, 256), 256, 0, s>>>(dw);
+    k_pair_class<<<blocks_for(d, P, kClassThreads), kClassThreads, 0, s>>>(dw);
     fork(1, side);
     k_narrow_class<PC_ANALYTIC><<<blocks_for(d, P, 128), 128, 0, side>>>(dw, p);
     k_boxes_axis<<<blocks_for(d, P, 128), 128, 0, side>>>(dw, p);
