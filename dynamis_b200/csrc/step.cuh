@@ -1988,6 +1988,9 @@ __device__ __forceinline__ void write_position_terms(const DeviceWorld& w, uint3
     w.srows.pdepth[i] = make_float4(depth[0], depth[1], depth[2], depth[3]);
 }
 
+// The guard's sixteen torque vectors would cost every block its registers, so guarded worlds have a
+// kernel of their own.
+template <bool kGuard>
 __global__ void __launch_bounds__(256) k_solve_prepare(DeviceWorld w, bool position_terms) {
     const uint32_t count = w.ctl[CTL_CONTACTS];
     const uint32_t cap = w.c_cap;
@@ -2032,7 +2035,7 @@ __global__ void __launch_bounds__(256) k_solve_prepare(DeviceWorld w, bool posit
             f3 arm_s = cross(rb[pi], normal);
             nm[pi] = count_f * (b.sf.inverse_mass + b.ss.inverse_mass) + dot(spread_f, arm_f) + dot(spread_s, arm_s);
         }
-        if ((w.solver_guard & DYN_SOLVER_GUARD_ROW_MASS) && pc >= 2u) guard_row_masses(b, normal, ra, rb, pc, count_f, nm);
+        if (kGuard && pc >= 2u) guard_row_masses(b, normal, ra, rb, pc, count_f, nm);
 #pragma unroll
         for (uint32_t pi = 0; pi < 4u; ++pi) if (pi < pc) {
             size_t o = (size_t)pi * cap + i;

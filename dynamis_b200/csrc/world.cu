@@ -850,7 +850,8 @@ void record_step(dyn_world* w, cudaStream_t s, uint32_t parity, bool timed, cons
         if (tape) k_tape_hot<<<blocks_for(d, N, 256), 256, 0, s>>>(dw, *tape, sub);
         k_integrate<<<blocks_for(d, N, 256), 256, 0, s>>>(dw, p);
         const uint32_t st = d->launch.solve_threads;
-        k_solve_prepare<<<blocks_for(d, C, st), st, 0, s>>>(dw, sub == 0u);
+        auto prepare = (w->solver_guard & DYN_SOLVER_GUARD_ROW_MASS) ? k_solve_prepare<true> : k_solve_prepare<false>;
+        prepare<<<blocks_for(d, C, st), st, 0, s>>>(dw, sub == 0u);
         if (joint_blocks) k_joint_prepare<<<blocks_for(d, dw.jcount, 128), 128, 0, s>>>(dw);
         if (sub == 0) {
             mark(ST_WARM);
