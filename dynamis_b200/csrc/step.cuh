@@ -2598,6 +2598,28 @@ __global__ void k_sleep(DeviceWorld w, dyn_step_params p) {
     }
 }
 
+// ---- checkpoints: the live entries of arrays that are kept at their capacity ----
+struct LivePart {
+    const char* from;
+    char* to;
+    uint32_t cap, counter, word;  // entries at most, the control word that counts them, bytes each (8 or 16)
+};
+struct LiveCopy {
+    LivePart part[24];
+    uint32_t parts;
+    const uint32_t* ctl;
+};
+// blockIdx.y is the part.
+__global__ void __launch_bounds__(256) k_copy_live(LiveCopy c) {
+    const LivePart& part = c.part[blockIdx.y];
+    const uint32_t n = min(c.ctl[part.counter], part.cap);
+    if (part.word == 16u) {
+        GRID_STRIDE(i, n) reinterpret_cast<uint4*>(part.to)[i] = __ldg(reinterpret_cast<const uint4*>(part.from) + i);
+    } else {
+        GRID_STRIDE(i, n) reinterpret_cast<uint2*>(part.to)[i] = __ldg(reinterpret_cast<const uint2*>(part.from) + i);
+    }
+}
+
 // ---- ABI state records <-> device layout (one contiguous copy each way) ----
 __global__ void k_unpack_states(DeviceWorld w, const dyn_body_state_record* __restrict__ in, uint32_t n) {
     GRID_STRIDE(i, n) {

@@ -1509,9 +1509,16 @@ static dyn_status step_once(dyn_world* w, float dt, bool taped) {
 // What a step reads that an earlier step wrote: the body rows and cold body fields, the contact set
 // the next step archives from (which of the two sets that is follows the parity), the counters and
 // control words.
+// The contact set and the frozen store are kept to their live prefix (CTL_ARCHIVED and CTL_RESTING
+// entries: nothing reads past it), by one kernel that reads the counts on the device: their capacity is
+// several times what a scene holds (1.5 GB of contacts for 262,144 bodies, 0.1 to 0.2 GB of them live).
+enum PartKind : uint32_t { PART_WHOLE, PART_CONTACTS, PART_FROZEN };
 struct CheckpointPart {
     void* ptr;
     size_t bytes;
+    PartKind kind = PART_WHOLE;
+    uint32_t slots = 1;  // point slots, each of the set's capacity
+    uint32_t word = 16;  // bytes per entry
 };
 static std::vector<CheckpointPart> checkpoint_parts(DeviceState* d) {
     DeviceWorld& dw = d->dw;
@@ -1520,12 +1527,13 @@ static std::vector<CheckpointPart> checkpoint_parts(DeviceState* d) {
     return {{dw.hot, N * sizeof(BodyHot)},        {dw.prev_pos, N * sizeof(float4)}, {dw.prev_rot, N * sizeof(float4)},
             {dw.force, N * sizeof(float4)},       {dw.torque, N * sizeof(float4)},   {dw.sleep_timer, N * sizeof(float)},
             {dw.wake_flags, N * sizeof(uint32_t)}, {dw.counters, 64 * sizeof(uint32_t)}, {dw.ctl, CTL_COUNT * sizeof(uint32_t)},
-            {arc.normal, C * sizeof(float4)},     {arc.rows, C * sizeof(uint4)},     {arc.mat, C * sizeof(float4)},
-            {arc.ids, C * sizeof(uint4)},         {arc.ids2, C * sizeof(uint4)},     {arc.extra, C * sizeof(float4)},
-            {arc.la, 4 * C * sizeof(float4)},     {arc.lb, 4 * C * sizeof(float4)},  {arc.acc, 4 * C * sizeof(float4)},
-            {arc.pos, 4 * C * sizeof(float4)},
-            {d->rest_ids[d->parity], (size_t)d->rest_cap * sizeof(uint4)},
-            {d->rest_slots[d->parity], (size_t)d->rest_cap * sizeof(uint2)},
+            {arc.normal, C * sizeof(float4), PART_CONTACTS},     {arc.rows, C * sizeof(uint4), PART_CONTACTS},
+            {arc.mat, C * sizeof(float4), PART_CONTACTS},        {arc.ids, C * sizeof(uint4), PART_CONTACTS},
+            {arc.ids2, C * sizeof(uint4), PART_CONTACTS},        {arc.extra, C * sizeof(float4), PART_CONTACTS},
+            {arc.la, 4 * C * sizeof(float4), PART_CONTACTS, 4},  {arc.lb, 4 * C * sizeof(float4), PART_CONTACTS, 4},
+            {arc.acc, 4 * C * sizeof(float4), PART_CONTACTS, 4}, {arc.pos, 4 * C * sizeof(float4), PART_CONTACTS, 4},
+            {d->rest_ids[d->parity], (size_t)d->rest_cap * sizeof(uint4), PART_FROZEN},
+            {d->rest_slots[d->parity], (size_t)d->rest_cap * sizeof(uint2), PART_FROZEN, 1, sizeof(uint2)},
             // the joints' accumulated impulses and broken flags (an empty part without joints)
             {dw.jruntime, (size_t)dw.jcount * sizeof(dyn_constraint_runtime_record)}};
 }
@@ -1539,33 +1547,52 @@ static void free_checkpoint(Checkpoint* c) {
     c->base = nullptr;
     c->bytes = 0;
 }
+// Copies every part between the world and the block at `base`, one way or the other, on the stream.
+static dyn_status copy_checkpoint(dyn_world* w, char* base, bool save) {
+    DeviceState* d = w->dev;
+    LiveCopy live{};
+    uint32_t most = 0;
+    char* at = base;
+    for (const CheckpointPart& part : checkpoint_parts(d)) {
+        char* world = static_cast<char*>(part.ptr);
+        if (part.ptr == d->dw.ctl) live.ctl = reinterpret_cast<const uint32_t*>(save ? world : at);
+        if (part.kind == PART_WHOLE) {
+            if (part.bytes) DYN_CUDA(cudaMemcpyAsync(save ? at : world, save ? world : at, part.bytes, cudaMemcpyDeviceToDevice, d->stream));
+        } else {
+            const size_t slot = part.bytes / part.slots;
+            const uint32_t cap = (uint32_t)(slot / part.word);
+            for (uint32_t k = 0; k < part.slots; ++k) {
+                LivePart& l = live.part[live.parts++];
+                l.from = (save ? world : at) + k * slot;
+                l.to = (save ? at : world) + k * slot;
+                l.cap = cap;
+                l.counter = part.kind == PART_CONTACTS ? CTL_ARCHIVED : CTL_RESTING;
+                l.word = part.word;
+            }
+            most = std::max(most, cap);
+        }
+        at += (part.bytes + 255u) & ~(size_t)255u;
+    }
+    k_copy_live<<<dim3(std::min(div_up(std::max(most, 1u), 256), d->sms * 2u), live.parts), 256, 0, d->stream>>>(live);
+    DYN_CUDA(cudaGetLastError());
+    return DYN_OK;
+}
 static dyn_status save_checkpoint(dyn_world* w, Checkpoint* c) {
     DeviceState* d = w->dev;
-    const std::vector<CheckpointPart> parts = checkpoint_parts(d);
-    const size_t bytes = checkpoint_bytes(parts);
+    const size_t bytes = checkpoint_bytes(checkpoint_parts(d));
     if (c->bytes != bytes) {
         free_checkpoint(c);
         DYN_CUDA(cudaMalloc(&c->base, bytes));
         c->bytes = bytes;
     }
-    char* at = static_cast<char*>(c->base);
-    for (const CheckpointPart& part : parts) {
-        if (part.bytes) DYN_CUDA(cudaMemcpyAsync(at, part.ptr, part.bytes, cudaMemcpyDeviceToDevice, d->stream));
-        at += (part.bytes + 255u) & ~(size_t)255u;
-    }
     c->parity = d->parity;
-    return DYN_OK;
+    return copy_checkpoint(w, static_cast<char*>(c->base), true);
 }
 static dyn_status restore_checkpoint(dyn_world* w, const Checkpoint& c) {
     DeviceState* d = w->dev;
     DYN_CUDA(cudaStreamSynchronize(d->stream));
     d->parity = c.parity;  // before listing the parts: the archived set follows the parity
-    const char* at = static_cast<const char*>(c.base);
-    for (const CheckpointPart& part : checkpoint_parts(d)) {
-        if (part.bytes) DYN_CUDA(cudaMemcpyAsync(part.ptr, at, part.bytes, cudaMemcpyDeviceToDevice, d->stream));
-        at += (part.bytes + 255u) & ~(size_t)255u;
-    }
-    return DYN_OK;
+    return copy_checkpoint(w, static_cast<char*>(c.base), false);
 }
 static void free_tape_buffers(TapeHost& t) {
     for (void* p : t.tape_allocs) cudaFree(p);
