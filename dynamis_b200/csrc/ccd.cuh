@@ -90,7 +90,8 @@ __device__ __forceinline__ SweepReach sweep_reach(const DeviceWorld& w, const Sw
 // A sweep is a chain of up to sixteen closest-point searches, each a chain of support evaluations:
 // its time is the latency of that chain, so a whole warp runs one direction of a pair and every
 // search spreads over its lanes (group_convex_hit). One thread per pair, its polytopes in local
-// memory, took 1,900 us on the 4,913-body pile with one CCD body in sixteen.
+// memory, took 1,898 us on the 4,913-body pile with one CCD body in sixteen, this takes 487 us behind
+// the list's rejection (635 us without it).
 using SweepLanes = Lanes<32>;
 struct SweepShared {
     SPt simplex[4];

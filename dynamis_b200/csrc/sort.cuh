@@ -153,7 +153,8 @@ __device__ __forceinline__ void scan_256(uint32_t a, uint32_t b, uint32_t* ea, u
 // the look-back's latency while few tiles run and by the scattered writes otherwise: a tile is 4096
 // keys (half as many look-backs as 2048), the digit totals' scan happens here and not in a launch of
 // its own, a thread looks back over eight tiles' words at a time, and the three arrays leave through
-// one staging buffer in turn, which keeps two blocks on an SM.
+// one staging buffer in turn, which keeps two blocks on an SM. 1M keys of two words with a payload, six
+// passes and the histogram: 116 -> 94 us.
 template <bool kTwoWords, bool kPayload>
 static __global__ void __launch_bounds__(kSortThreads, 2)
     k_onesweep(const uint32_t* __restrict__ key_in, const uint32_t* __restrict__ other_in,

@@ -724,7 +724,6 @@ void record_step(dyn_world* w, cudaStream_t s, uint32_t parity, bool timed, cons
     DeviceState* d = w->dev;
     DeviceWorld dw = d->dw;
     if (parity) std::swap(dw.cur, dw.arc);
-    dw.solver_guard = w->solver_guard;
     if (tape) {
         dw.tape = TapeWrites{tape->slot, tape->relay, tape->vel, tape->acc, tape->res, tape->cnt,
                              tape->substeps, tape->iterations, tape->piterations, tape->n, tape->c};
