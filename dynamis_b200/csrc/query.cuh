@@ -563,13 +563,20 @@ __device__ __forceinline__ void write_hit(const DeviceWorld& w, const QHit& hit,
     *out = r;
 }
 
-// Can a ray of this query reach the box at all? Every ray test is analytic, so a ray that clears the
-// box by more than the tests' rounding meets nothing in it. The largest rounding is that of a
-// quadratic's discriminant, about 5e-7 of the squared distance, which answers a miss by up to 7e-4 of
-// the distance as a hit: the box is grown by three times that and a millimetre.
+// Can a ray reach the box at all? Asked for the colliders whose class record says kClassBoxedRays only
+// (unscaled spheres, cuboids, capsules and cylinders); the others always go on to their test: a
+// scaled frame's test answers hits past the ray's end, and a triangle's is unbounded near its plane.
+// For the four, with u = 2^-24 and a unit heading, a test that answers a hit at t has its point o + t d
+//   * for a quadratic (sphere, capsule, a cylinder's side): within sqrt(r^2 + 21 u |offset|^2) of the
+//     centre or axis, the discriminant's rounding, so at most 1.2e-3 |offset| outside;
+//   * for a slab or a cap: within 100 u of the lengths involved (rotations included; a rotation that
+//     is a unit only to 1e-4 adds 4e-4 of them);
+// and the box and centres are rounded at world coordinates, 4 u of these. `far` bounds every such
+// length, so the slack holds all of it, with the millimetre left for an axis the ray hardly moves on.
 __device__ __forceinline__ bool ray_meets(f3 origin, f3 heading, float extent, f3 mn, f3 mx) {
     const f3 far = vmax(vabs(mn - origin), vabs(mx - origin));
-    const float slack = 1e-3f + 2e-3f * (far.x + far.y + far.z);
+    const f3 world = vmax(vabs(mn), vabs(mx)) + vabs(origin);
+    const float slack = 1e-3f + 2e-3f * (far.x + far.y + far.z) + 1e-6f * (world.x + world.y + world.z);
     float near_t = -slack, far_t = extent + slack;
     for (uint32_t axis = 0; axis < 3u; ++axis) {
         const float o = comp(origin, axis), d = comp(heading, axis);
@@ -646,7 +653,7 @@ __device__ __forceinline__ QHit warp_resolve(const Lanes<32>& L, const DeviceWor
 // three of its four warps waiting at barriers for the one that tested hits (7 of 16 cycles per
 // instruction), and tested candidates where they lay among their duplicates (8 of 32 threads per
 // instruction): here the distinct ones are packed first, and a ray's candidates that its box test
-// rules out are dropped before the sort. A query with more candidates than the warp holds goes to
+// rules out (ray_meets) are dropped before the sort. A query with more candidates than the warp holds goes to
 // k_scene_query_large.
 __global__ void __launch_bounds__(kQueryThreads) k_scene_query(DeviceWorld w, dyn_query_record* queries, dyn_query_hit_record* hits,
                                                                uint32_t count, uint32_t* __restrict__ large) {
@@ -672,12 +679,14 @@ __global__ void __launch_bounds__(kQueryThreads) k_scene_query(DeviceWorld w, dy
         const DAabb box = query_box(w, q);
         const bool is_ray = q.kind == DYN_QUERY_RAY;
         const f3 origin = q_origin(q), heading = is_ray ? normalize(q_direction(q)) : s3(0.0f);
+        const bool drops = is_ray && fabsf(dot(heading, heading) - 1.0f) < 1e-3f;
         auto push = [&](const GEntry& e) {
             const uint32_t seen = atomicAdd(&sh.seen, 1u);
             if (seen >= DYN_QUERY_CANDIDATES) return;
-            if (is_ray && !ray_meets(origin, heading, q.extent, e.mn, e.mx)) return;
+            const uint32_t slot = e.info & DYN_ENTRY_INDEX_MASK;
+            if (drops && !ray_meets(origin, heading, q.extent, e.mn, e.mx) && (w.c_class[slot].w & kClassBoxedRays)) return;
             const uint32_t at = atomicAdd(&sh.kept, 1u);
-            if (at < kWarpCandidates) sh.candidates[at] = e.info & DYN_ENTRY_INDEX_MASK;
+            if (at < kWarpCandidates) sh.candidates[at] = slot;
         };
         uint32_t occupied = (q.filters.targets & DYN_QUERY_TARGET_COLLIDERS) != 0u ? levels : 0u;
 #pragma unroll 1

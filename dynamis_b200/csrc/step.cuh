@@ -223,6 +223,21 @@ __global__ void k_begin(DeviceWorld w, dyn_step_params p) {
 
 __device__ __forceinline__ float grid_extent_of(f3 mn, f3 mx) { return wmax(wmax(mx.x - mn.x, mx.y - mn.y), mx.z - mn.z); }
 
+// A collider whose rays meet it only where they meet its box (ray_meets, query.cuh): a sphere, cuboid,
+// capsule or cylinder in its own frame, with a unit rotation and sizes that are not degenerate. The
+// caller adds "unscaled": a scaled frame's ray test measures the extent in that frame's lengths and
+// answers hits past the ray's end.
+constexpr uint32_t kClassBoxedRays = 0x400u;  // in c_class[].w
+__device__ __forceinline__ bool rays_stay_in_box(const WShape& s) {
+    const float4 q = s.rotation;
+    const float square = q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
+    if (!(fabsf(square - 1.0f) < 1e-4f)) return false;
+    if (s.kind == DYN_SHAPE_SPHERE) return s.radius >= 0.0f;
+    if (s.kind == DYN_SHAPE_CUBOID) return s.half_extents.x >= 0.0f && s.half_extents.y >= 0.0f && s.half_extents.z >= 0.0f;
+    if (s.kind == DYN_SHAPE_CAPSULE || s.kind == DYN_SHAPE_CYLINDER) return s.radius >= 0.0f && s.half_height >= 1e-6f;
+    return false;
+}
+
 // broadphase_aabb.wgsl:11-62 (core.wgsl:109-126 for the grid resolution)
 __global__ void k_aabb(DeviceWorld w, dyn_step_params p) {
     GRID_STRIDE(i, w.k) {
@@ -233,15 +248,16 @@ __global__ void k_aabb(DeviceWorld w, dyn_step_params p) {
         }
         DBody b = load_dbody(w.hot, owner);
         DColl c = load_dcoll(w, i);
+        WShape s = world_shape(b.position, b.orientation, c);
         {  // what k_pair_class asks of this collider, in one record (nothing it reads changes before it runs)
             const uint4 id = w.ident[owner];
             const uint2 f = w.c_filter[i];
             const bool unscaled = veq(c.scale, s3(1.0f));
             w.c_class[i] = make_uint4(owner, f.x != DYN_NO_COLLISION_FILTER ? f.x : id.z,
                                       f.y != DYN_NO_COLLISION_FILTER ? f.y : id.w,
-                                      c.kind | (moves(b.inverse_mass, b.flags) ? 0x100u : 0u) | (unscaled ? 0x200u : 0u));
+                                      c.kind | (moves(b.inverse_mass, b.flags) ? 0x100u : 0u) | (unscaled ? 0x200u : 0u) |
+                                          (unscaled && rays_stay_in_box(s) ? kClassBoxedRays : 0u));
         }
-        WShape s = world_shape(b.position, b.orientation, c);
         DAabb tight = world_aabb(w, s);
         WShape up = s;
         up.rotation = make_float4(0.0f, 0.0f, 0.0f, 1.0f);

@@ -115,3 +115,66 @@ def test_queries_on_a_formed_pile():
     gq, _ = compare(w, random_queries(rng, 96, 10.0, 0))
     assert gq["count"].sum() > 50
     w.close()
+
+
+SCALES = [(1, 0.5, 1), (0.5, 0.5, 0.5), (4, 0.25, 1), (0.25, 3, 0.5)]
+
+
+def scaled_targets(crowd):
+    """Scaled round colliders 20 m apart, a sphere that sets the grid's cell, and around the first
+    collider's ray `crowd` spheres whose boxes hold the ray but which it misses."""
+    bodies = [static_sphere(0.495, (0, 0, -20))]
+    for i, (kind, scale) in enumerate((k, s) for k in (R.SHAPE_SPHERE, R.SHAPE_CAPSULE, R.SHAPE_CYLINDER) for s in SCALES):
+        size = dict(radius=0.5) if kind == R.SHAPE_SPHERE else dict(radius=0.25, half_height=0.25)
+        bodies.append(dict(shape=kind, scale=scale, mass=0.0, position=(0.6 + 20 * i, 0.5, 0.6), **size))
+    rng = np.random.default_rng(crowd)
+    for _ in range(crowd):
+        x, z = 0.2 + rng.uniform(-0.04, 0.04, 2)
+        bodies.append(static_sphere(0.495, (x, rng.uniform(2.0, 9.0), z)))
+    return make(bodies)[0]
+
+
+@pytest.mark.parametrize("crowd", [0, 700])
+def test_rays_past_their_end_into_scaled_shapes_match_the_oracle(crowd):
+    # a scaled shape's test takes the extent in its own frame's lengths, so where a scale is below 1
+    # along the ray it answers a hit past the ray's end; 700 boxes around a ray put it past the 512
+    # candidates a warp holds
+    w = scaled_targets(crowd)
+    queries = [R.ray_query((0.6 + 20 * i, 10.0, 0.6), (0.0, -1.0, 0.0), float(extent), R.query_filter(max_hits=4))
+               for i in range(3 * len(SCALES)) for extent in np.linspace(7.6, 9.8, 12)]
+    gq, gh = compare(w, queries)
+    past = [gh[r["hit_base"]]["distance"] > r["extent"] for r in gq if r["count"]]
+    assert sum(past) > 20  # the case is met
+    w.close()
+
+
+@pytest.mark.parametrize("offset", [0.0, 300.0, 40000.0])
+def test_grazing_rays_match_the_oracle(offset):
+    # rays that pass within rounding of each shape's surface, near and far from it and from the world's origin
+    rng = np.random.default_rng(int(offset))
+    bodies = []
+    for i in range(24):
+        quat = rng.normal(size=4)
+        quat /= np.linalg.norm(quat)
+        common = dict(mass=0.0, position=(offset + 8.0 * i, offset, -offset), orientation=quat)
+        bodies.append([dict(shape=R.SHAPE_SPHERE, radius=0.7, **common), dict(shape=R.SHAPE_CUBOID, half_extents=(0.3, 0.5, 0.7), **common),
+                       dict(shape=R.SHAPE_CAPSULE, radius=0.3, half_height=0.6, **common),
+                       dict(shape=R.SHAPE_CYLINDER, radius=0.4, half_height=0.5, **common)][i % 4])
+    w, _ = make(bodies)
+    queries = []
+    for _ in range(1200):
+        spec = bodies[int(rng.integers(0, 24))]
+        centre = np.asarray(spec["position"], np.float64)
+        d = rng.normal(size=3)
+        d /= np.linalg.norm(d)
+        side = np.cross(d, rng.normal(size=3))
+        side /= np.linalg.norm(side)
+        reach = {R.SHAPE_SPHERE: 0.7, R.SHAPE_CAPSULE: 0.3, R.SHAPE_CYLINDER: 0.4}.get(spec["shape"], 0.5)
+        miss = reach * (1.0 + rng.normal() * 10.0 ** rng.uniform(-7, -1))
+        back = 10.0 ** rng.uniform(0, 2.5)
+        # a quarter of them end at the shape
+        extent = back if rng.random() < 0.25 else 2 * back
+        queries.append(R.ray_query(centre + side * miss - d * back, d, float(extent), R.query_filter(max_hits=8)))
+    gq, _ = compare(w, queries)
+    assert 100 < gq["count"].astype(bool).sum() < len(queries)
+    w.close()
