@@ -161,8 +161,13 @@ __device__ SweepHit rigid_sweep(const SweepLanes& L, const DeviceWorld& w, const
 // sweep's start bounds the distance the search would report from below (narrow.cuh, gjk_phase), and the
 // approach it is divided by is at most the relative travel plus the turning of both shapes. When the
 // gap exceeds that by more than rounding, the first step of rigid_sweep passes the end of the step
-// whatever its normal. Planes are left to the sweep, whose gap to them is one support evaluation.
-constexpr float kSweepRejectTolerance = 1e-3f;
+// whatever its normal. Rounding: a support point carries two roundings of its world coordinates
+// (2 x 2^-24 of each), the gap here and the search's take two points each, so the two gaps differ by
+// at most 5e-7 of a centre's length beside what the millimetre holds; the term takes 4e-7 of both
+// centres' coordinates. Without it hits were dropped from some tens of kilometres out (in 1M pairs at
+// the end of their reach, 21 at 65 km and 304 at 260 km; none with it). Planes are left to the
+// sweep, whose gap to them is one support evaluation.
+constexpr float kSweepRejectTolerance = 1e-3f, kSweepRejectCoordinates = 4e-7f;
 __device__ __forceinline__ bool sweep_cannot_reach(const DeviceWorld& w, const SweptBody& moving, const DColl& mc,
                                                    const SweptBody& other, const DColl& oc) {
     if (mc.kind == DYN_SHAPE_PLANE || oc.kind == DYN_SHAPE_PLANE) return false;
@@ -180,7 +185,9 @@ __device__ __forceinline__ bool sweep_cannot_reach(const DeviceWorld& w, const S
                                        : world_shape(other.body.position, other.body.orientation, oc);
     const f3 axis = fixed.center - free.center;
     const float gap = -dot(support(w, free, axis) - support(w, fixed, -axis), axis);
-    return gap > (reach * (1.0f + kSweepRejectTolerance) + kSweepRejectTolerance) * length(axis);
+    const f3 at = vabs(free.center) + vabs(fixed.center);
+    const float rounding = kSweepRejectTolerance + kSweepRejectCoordinates * (at.x + at.y + at.z);
+    return gap > (reach * (1.0f + kSweepRejectTolerance) + rounding) * length(axis);
 }
 
 // ccd_sweep.wgsl:188-211 (the pairs are unique, so the sorted list's duplicate check has nothing to

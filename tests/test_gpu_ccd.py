@@ -149,3 +149,65 @@ def test_a_fast_heap_of_every_shape_lands_like_the_oracle():
     # swept (ccd_sweep.wgsl:130-133), so no bound on every body is asserted, only the parity above
     assert np.sum(o.states()["position"][:, 1] > -1.0) >= len(scene.bodies) - 3
     w.close()
+
+
+def extent_along(shape, size, quats, axis):
+    """The reach of each rotated shape along its row of `axis`."""
+    local = np.stack([quat_rotate(q * (-1, -1, -1, 1), a) for q, a in zip(quats, axis)])
+    if shape == "sphere":
+        return size[:, 0]
+    if shape == "box":
+        return np.abs(local * size).sum(axis=1)
+    return np.abs(local[:, 1]) * size[:, 1] + size[:, 0]  # capsule
+
+
+@pytest.mark.parametrize("offset", [0.0, 260000.0])
+def test_sweeps_that_just_reach_match_the_oracle_far_from_the_origin(offset):
+    # pairs whose travel ends within a percent of the gap between them, alone and so without contacts:
+    # a direction is left out of the sweep only when rounding at its coordinates cannot make it arrive
+    from test_ccd import R, STATIC
+    rng = np.random.default_rng(11)
+    n = 16000
+    side = int(np.ceil(n ** (1 / 3)))
+    i = np.arange(n)
+    at = np.stack([i % side, i // side % side, i // side // side], 1) * 10.0 + offset * np.array([1.0, -0.7, 0.4])
+    at = at.astype(np.float32).astype(np.float64)
+    axis = rng.normal(size=(n, 3))
+    axis /= np.linalg.norm(axis, axis=1, keepdims=True)
+    kinds = np.maximum(rng.integers(-5, 3, (2, n)), 0)  # mostly spheres, whose gap the centre axis gives exactly
+    sizes = rng.uniform(0.15, 0.6, (2, n, 3))
+    quats = rng.normal(size=(2, n, 4))
+    quats /= np.linalg.norm(quats, axis=2, keepdims=True)
+    reach = np.zeros((2, n))
+    for s in range(2):
+        for k, name in enumerate(("sphere", "box", "capsule")):
+            rows = kinds[s] == k
+            reach[s, rows] = extent_along(name, sizes[s, rows], quats[s, rows], axis[rows])
+    apart = reach.sum(axis=0) + rng.uniform(0.4, 1.5, n)
+    target = (at + axis * apart[:, None]).astype(np.float32)
+    between = np.asarray(target, np.float64) - at
+    gap = np.linalg.norm(between, axis=1) - reach.sum(axis=0)
+    travel = axis * (gap * (1.0 + rng.normal(0.0, 0.01, n)))[:, None]
+    bodies, colliders = R.body_defaults(2 * n), R.collider_defaults(2 * n)
+    bodies["position"] = np.concatenate([at, target])
+    bodies["orientation"] = np.concatenate(quats)
+    bodies["velocity"][:n] = travel / DT
+    bodies["ccd"][:n] = 1
+    bodies["mass"][n:] = 0.0
+    kind, size = np.concatenate(kinds), np.concatenate(sizes)
+    colliders["shape"] = np.choose(kind, [R.SHAPE_SPHERE, R.SHAPE_CUBOID, R.SHAPE_CAPSULE])
+    colliders["half_extents"] = size
+    colliders["radius"], colliders["half_height"] = size[:, 0], size[:, 1]
+    w = World(**STATIC, capacity={"pairs": 1 << 21})
+    w.spawn(bodies, colliders)
+    oracle = oracle_from_world(w, DT)
+    w.step(DT)
+    oracle.step(DT)
+    w.wait()
+    got, want = w.read_states(), oracle.states()
+    moved = np.linalg.norm(want["velocity"][:n], axis=1) < 0.9 * np.linalg.norm(travel / DT, axis=1)
+    assert 0.1 * n < moved.sum() < 0.9 * n  # many arrive, many do not
+    for name in ("position", "orientation", "velocity", "angular_velocity"):
+        differ = np.any(got[name] != want[name], axis=1)
+        assert not differ.any(), f"{name}: {differ.sum()} bodies differ, first {np.nonzero(differ)[0][:4]}"
+    w.close()
