@@ -2639,8 +2639,9 @@ struct LivePart {
     char* to;
     uint32_t cap, counter, word;  // entries at most, the control word that counts them, bytes each (8 or 16)
 };
+constexpr uint32_t kLiveParts = 24u;  // of one launch: a contact set's 6 columns and 4 x 4 point slots, a frozen store's 2
 struct LiveCopy {
-    LivePart part[24];
+    LivePart part[kLiveParts];
     uint32_t parts;
     const uint32_t* ctl;
 };

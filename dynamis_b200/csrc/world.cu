@@ -1549,30 +1549,42 @@ static void free_checkpoint(Checkpoint* c) {
 // Copies every part between the world and the block at `base`, one way or the other, on the stream.
 static dyn_status copy_checkpoint(dyn_world* w, char* base, bool save) {
     DeviceState* d = w->dev;
+    const std::vector<CheckpointPart> parts = checkpoint_parts(d);
+    auto advance = [](char* at, const CheckpointPart& part) { return at + ((part.bytes + 255u) & ~(size_t)255u); };
     LiveCopy live{};
-    uint32_t most = 0;
     char* at = base;
-    for (const CheckpointPart& part : checkpoint_parts(d)) {
+    for (const CheckpointPart& part : parts) {  // the counts come from the side that is copied
+        if (part.ptr == d->dw.ctl) live.ctl = reinterpret_cast<const uint32_t*>(save ? static_cast<char*>(part.ptr) : at);
+        at = advance(at, part);
+    }
+    uint32_t most = 0;
+    auto launch = [&] {
+        k_copy_live<<<dim3(std::min(div_up(std::max(most, 1u), 256), d->sms * 2u), live.parts), 256, 0, d->stream>>>(live);
+        live.parts = 0u;
+        most = 0u;
+    };
+    at = base;
+    for (const CheckpointPart& part : parts) {
         char* world = static_cast<char*>(part.ptr);
-        if (part.ptr == d->dw.ctl) live.ctl = reinterpret_cast<const uint32_t*>(save ? world : at);
         if (part.kind == PART_WHOLE) {
             if (part.bytes) DYN_CUDA(cudaMemcpyAsync(save ? at : world, save ? world : at, part.bytes, cudaMemcpyDeviceToDevice, d->stream));
         } else {
             const size_t slot = part.bytes / part.slots;
             const uint32_t cap = (uint32_t)(slot / part.word);
             for (uint32_t k = 0; k < part.slots; ++k) {
+                if (live.parts == kLiveParts) launch();
                 LivePart& l = live.part[live.parts++];
                 l.from = (save ? world : at) + k * slot;
                 l.to = (save ? at : world) + k * slot;
                 l.cap = cap;
                 l.counter = part.kind == PART_CONTACTS ? CTL_ARCHIVED : CTL_RESTING;
                 l.word = part.word;
+                most = std::max(most, cap);
             }
-            most = std::max(most, cap);
         }
-        at += (part.bytes + 255u) & ~(size_t)255u;
+        at = advance(at, part);
     }
-    k_copy_live<<<dim3(std::min(div_up(std::max(most, 1u), 256), d->sms * 2u), live.parts), 256, 0, d->stream>>>(live);
+    if (live.parts) launch();
     DYN_CUDA(cudaGetLastError());
     return DYN_OK;
 }
