@@ -2450,6 +2450,7 @@ DYN_API dyn_status dyn_query(dyn_world* w, dyn_query_record* queries, uint32_t n
         DYN_CUDA(cudaStreamSynchronize(d->stream));
         if (d->hit_buf) cudaFree(d->hit_buf);
         d->hit_buf = nullptr;
+        d->hit_cap = 0;  // a failed allocation leaves no capacity behind
         DYN_CUDA(cudaMalloc(&d->hit_buf, (size_t)std::max<uint64_t>(base, 1) * sizeof(dyn_query_hit_record)));
         d->hit_cap = (uint32_t)std::max<uint64_t>(base, 1);
     }
