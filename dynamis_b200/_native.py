@@ -50,6 +50,7 @@ SIGNATURES = {
     "dyn_debug_pairs": (I32, [P, P, P, U32, PU32]),
     "dyn_debug_contacts": (I32, [P, P, U32, PU32]),
     "dyn_debug_islands": (I32, [P, P, U32, PU32]),
+    "dyn_debug_paths": (I32, [P, P]),
     "dyn_debug_resting": (I32, [P, P, U32, PU32]),
     "dyn_query": (I32, [P, P, U32, P, U32]),
     "dyn_hull_triangles": (I32, [P, U32, P, U32, PU32]),

@@ -79,7 +79,8 @@ enum Ctl : uint32_t {
     CTL_CCD_NEXT = 25,       // the next of them
     CTL_BOX_HITS = 26,       // touching box pairs queued for the manifold
     CTL_QUERY_NEXT = 27,     // a query batch's next query (in the query's own control words)
-    CTL_QUERY_LARGE = 28,    // its queries left to k_scene_query_large
+    CTL_QUERY_LARGE = 28,    // its queries that the warps hand on to blocks
+    CTL_QUERY_LARGE_NEXT = 29,  // the next of them, or of a batch that goes to blocks
     CTL_COUNT = 32
 };
 

@@ -951,101 +951,6 @@ __device__ __forceinline__ bool gjk_repeats(const float* lam, uint32_t count, f3
            __float_as_uint(newest.z) == __float_as_uint(support_point.z);
 }
 
-// convex.wgsl:464-521 then 584-618
-__device__ Hit convex_hit(const DeviceWorld& w, const WShape& first, const WShape& second) {
-    SPt s[4];
-    uint32_t count = 0;
-    float rdist = 0.0f;
-    f3 rpa = first.center, rpb = second.center;
-    f3 rnormal = sign_normalize(second.center - first.center);
-    bool rpen = false;
-    f3 dir = second.center - first.center;
-    if (length(dir) < 1e-8f) dir = mk3(1.0f, 0.0f, 0.0f);
-    s[0] = support_pair(w, first, second, dir);
-    count = 1;
-    SRes cl = simplex_closest(s, count);
-    float tiny = 1e-4f * wmin(shape_scale(first), shape_scale(second));
-    for (uint32_t iter = 0; iter < kGjkIterations; ++iter) {
-        if (cl.pen || length(cl.v) < tiny) {
-            while (count < 4u) {
-                f3 d = simplex_expand_dir(s, count);
-                s[count] = support_pair(w, first, second, d);
-                count += 1;
-            }
-            rpen = true;
-            rdist = 0.0f;
-            rpa = cl.pa;
-            rpb = cl.pb;
-            break;
-        }
-        SPt sp = support_pair(w, first, second, -cl.v);
-        if (dot(sp.w, -cl.v) <= dot(cl.v, -cl.v) + 1e-4f * wmax(1.0f, dot(cl.v, cl.v))) {
-            rdist = length(cl.v);
-            rpa = cl.pa;
-            rpb = cl.pb;
-            if (rdist > 1e-6f) rnormal = sign_normalize(cl.pb - cl.pa);
-            break;
-        }
-        const bool repeats = gjk_repeats(cl.lam, count, s[count - 1u].w, sp.w);
-        // simplex_reduce
-        SPt kept[4];
-        uint32_t kc = 0;
-        for (uint32_t i = 0; i < 4; ++i) {
-            if (cl.lam[i] > 1e-6f) kept[kc++] = s[i];
-        }
-        if (kc == 0u) {
-            kept[0] = s[0];
-            kc = 1;
-        }
-        for (uint32_t i = 0; i < kc; ++i) s[i] = kept[i];
-        count = kc;
-        // simplex_holds
-        float span = shape_scale(second);
-        float tol = (1e-5f * span) * (1e-5f * span);
-        bool holds = false;
-        for (uint32_t i = 0; i < count; ++i) {
-            f3 off = s[i].w - sp.w;
-            if (dot(off, off) <= tol) holds = true;
-        }
-        if (holds) {
-            rdist = length(cl.v);
-            rpa = cl.pa;
-            rpb = cl.pb;
-            if (rdist > 1e-6f) rnormal = sign_normalize(cl.pb - cl.pa);
-            break;
-        }
-        s[count] = sp;
-        count += 1;
-        if (repeats) break;
-        cl = simplex_closest(s, count);
-    }
-    if (!rpen) {
-        EpaOut probe = penetration_probe(w, first, second, s, count, true);
-        if (probe.depth > 0.0f) {
-            f3 normal = probe.normal;
-            if (dot(normal, second.center - first.center) < 0.0f) normal = -normal;
-            return Hit{-probe.depth, (rpa + rpb) * 0.5f, normal};
-        }
-        if (rdist > 0.0f) return Hit{rdist, (rpa + rpb) * 0.5f, rnormal};
-        return Hit{3.402823466e38f, s3(0.0f), s3(0.0f)};
-    }
-    EpaOut epa = epa_tetrahedron(w, first, second, s);
-    Hit result;
-    if (epa.valid && epa.depth > 0.0f && epa.depth < 3.402823466e38f && length(epa.normal) > 0.5f
-        && epa.depth < support_projection_depth(w, first, second, epa.normal) + 0.1f * wmin(shape_scale(first), shape_scale(second))) {
-        f3 pa = support(w, first, epa.normal);
-        f3 pb = support(w, second, -epa.normal);
-        result = Hit{-epa.depth, (pa + pb) * 0.5f, epa.normal};
-    } else {
-        EpaOut probe = penetration_probe(w, first, second, s, count);
-        f3 pa = support(w, first, probe.normal);
-        f3 pb = support(w, second, -probe.normal);
-        result = Hit{-probe.depth, (pa + pb) * 0.5f, probe.normal};
-    }
-    if (dot(result.normal, second.center - first.center) < 0.0f) result.normal = -result.normal;
-    return result;
-}
-
 // ---- the convex path in three phases (results identical to convex_hit) ----
 //
 // Phase 1, one thread per pair: GJK (convex.wgsl:464-521) and, for separated shapes, the

@@ -2,7 +2,7 @@
 // convex sweeps against the colliders (crates/dynamis-shader/shaders/scene_cast.wgsl:1-534 for the
 // candidate walk and the hit selection; scene.wgsl:1-258, 259-320, 813-873 for the hit tests).
 //
-// One warp per query, or one block where a warp cannot hold its candidates. They are the colliders with an entry in the grid cells the
+// A team of one or four warps per query (k_scene_query). The candidates are the colliders with an entry in the grid cells the
 // query's box covers, level by level (grid_index.wgsl:289-388: a level whose cells under the box
 // number more than GRID_WALK_CELLS is scanned whole, entries tested against the box; otherwise its
 // cells are looked up one by one), at most QUERY_CANDIDATES of them (more set the overflow flag).
@@ -451,12 +451,6 @@ __device__ __forceinline__ void finish_inside(const DeviceWorld& w, const dyn_qu
         geom_normal(w, q, world, hit);
     }
 }
-__device__ QHit resolve_hit(const DeviceWorld& w, const dyn_query_record& q, const WShape& world, bool whole) {
-    Resolved r = resolve_lane(w, q, world, whole);
-    if (r.inside) finish_inside(w, q, world, convex_hit(w, query_probe(q, q_origin(q)), world), whole, &r.hit);
-    return r.hit;
-}
-
 // body_passes (scene_cast.wgsl:196-222) and collider_filter_query (core.wgsl:285-291)
 __device__ bool query_passes(const DeviceWorld& w, const dyn_query_record& q, uint32_t slot) {
     const uint32_t row = w.c_owner[slot];
@@ -502,44 +496,6 @@ __device__ __forceinline__ uint32_t hit_key(float distance) {
     return (bits & 0x80000000u) != 0u ? ~bits : (bits | 0x80000000u);
 }
 
-// Bitonic sort of `width` (a power of two) values in shared memory, ascending, by the whole block.
-template <typename T>
-__device__ void block_bitonic(T* values, uint32_t width) {
-    for (uint32_t k = 2u; k <= width; k <<= 1) {
-        for (uint32_t j = k >> 1; j > 0u; j >>= 1) {
-            for (uint32_t index = threadIdx.x; index < width; index += blockDim.x) {
-                const uint32_t other = index ^ j;
-                if (other > index) {
-                    const bool ascending = (index & k) == 0u;
-                    const T a = values[index], b = values[other];
-                    if (ascending ? a > b : a < b) {
-                        values[index] = b;
-                        values[other] = a;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-}
-
-struct QueryShared {
-    uint32_t candidates[DYN_QUERY_CANDIDATES];
-    unsigned long long keys[DYN_QUERY_CANDIDATES];
-    uint32_t candidate_count;
-    uint32_t overflow;
-    uint32_t hit_total;
-};
-
-__device__ __forceinline__ void push_candidate(QueryShared& sh, uint32_t slot) {
-    const uint32_t at = atomicAdd(&sh.candidate_count, 1u);
-    if (at >= DYN_QUERY_CANDIDATES) {
-        sh.overflow = 1u;
-        return;
-    }
-    sh.candidates[at] = slot;
-}
-
 __device__ __forceinline__ WShape collider_shape(const DeviceWorld& w, uint32_t slot) {
     const DBody b = load_dbody(w.hot, w.c_owner[slot]);
     return world_shape(b.position, b.orientation, load_dcoll(w, slot));
@@ -561,6 +517,18 @@ __device__ __forceinline__ void write_hit(const DeviceWorld& w, const QHit& hit,
     r.normal[2] = hit.normal.z;
     r.surface = DYN_NO_SURFACE;  // hull triangles carry no surface (crates/dynamis-world/src/shape_pool.rs:557-580)
     *out = r;
+}
+
+// Is this entry, met in `cell`, a repeat of a collider whose entry in an earlier one of the query's
+// cells (from `lo`) is met too? A collider's entries are the cells of its box, two an axis at most; the
+// offset bits tell the lowest from the second. An entry met in another cell than its own (their hashes
+// meet) is no repeat, nor is any of a box that spans more (its coordinates are not finite).
+__device__ __forceinline__ bool entry_again(const GEntry& e, float cs, I3 lo, I3 cell) {
+    const uint32_t bits = (e.info & DYN_ENTRY_CELL_MASK) >> DYN_ENTRY_CELL_SHIFT;
+    if (!(((bits & 1u) && cell.x != lo.x) || ((bits & 2u) && cell.y != lo.y) || ((bits & 4u) && cell.z != lo.z))) return false;
+    const I3 a = floor_div(e.mn, cs), b = floor_div(e.mx, cs);
+    if ((long long)b.x - a.x > 1 || (long long)b.y - a.y > 1 || (long long)b.z - a.z > 1) return false;
+    return same_cell(I3{a.x + (int)(bits & 1u), a.y + (int)((bits >> 1) & 1u), a.z + (int)((bits >> 2) & 1u)}, cell);
 }
 
 // Can a ray reach the box at all? Asked for the colliders whose class record says kClassBoxedRays only
@@ -592,46 +560,76 @@ __device__ __forceinline__ bool ray_meets(f3 origin, f3 heading, float extent, f
     return !(near_t > far_t + slack);
 }
 
-// A warp's queries keep their candidates in 6 KB of shared memory and a polytope in 4, so sixteen run
-// on an SM.
+// A query belongs to a team of warps: a single warp where a batch fills the chip with warps, a block
+// where it does not or where the query has more candidates than a warp's space holds.
 constexpr uint32_t kWarpCandidates = 512u;
-struct QueryWarpShared {
+// Where the lines lie (32,768-body pile; us a call, host included). A batch of up to two queries an SM
+// goes to blocks (warps / blocks): 256 box sweeps 5,377 / 2,708, rays of 60 m 2,883 / 1,795, box
+// overlaps 1,091 / 672, short rays 530 / 450; 1,024 short rays 733 / 959. Up to eight an SM a query whose
+// box covers more than kWideCells cells, all levels together, goes to a block too, since one warp's
+// walk and search would outlast the batch (warps alone / handed on): 512 rays of 60 m 3,262 / 1,758,
+// 512 box sweeps 5,566 / 4,976, 1,024 rays of 60 m 3,438 / 2,827, 1,024 long box sweeps 20,462 / 15,789,
+// 1,024 short box sweeps 7,702 / 9,222; 2,048 of these 16,330 / 17,215.
+constexpr uint32_t kBlockQueriesPerSm = 2u, kWideQueriesPerSm = 8u, kWideCells = 256u;
+// What a warp's penetration search takes (group_convex_hit).
+struct QuerySearch {
     EpaWarpShared epa;
     SPt simplex[4];
-    unsigned long long keys[kWarpCandidates];
-    uint32_t candidates[kWarpCandidates];
-    uint32_t seen, kept;  // candidates met, and those of them a ray can meet
 };
-// block_bitonic by one warp.
-template <typename T>
-__device__ __forceinline__ void warp_bitonic(T* values, uint32_t width) {
-    const uint32_t lane = threadIdx.x & 31u;
-#pragma unroll 1
-    for (uint32_t k = 2u; k <= width; k <<= 1) {
-#pragma unroll 1
-        for (uint32_t j = k >> 1; j > 0u; j >>= 1) {
-#pragma unroll 1
-            for (uint32_t index = lane; index < width; index += 32u) {
-                const uint32_t other = index ^ j;
-                if (other > index) {
-                    const bool ascending = (index & k) == 0u;
-                    const T a = values[index], b = values[other];
-                    if (ascending ? a > b : a < b) {
-                        values[index] = b;
-                        values[other] = a;
-                    }
-                }
-            }
+template <uint32_t kWarps>
+struct QueryTeam {
+    static constexpr uint32_t kThreads = 32u * kWarps;
+    static constexpr uint32_t kCap = kWarps == 1u ? kWarpCandidates : DYN_QUERY_CANDIDATES;
+    QuerySearch search[kWarps];
+    unsigned long long keys[kCap];
+    uint32_t candidates[kCap];
+    uint32_t next;            // the query
+    uint32_t seen, kept;      // entries met, and those of them kept as candidates
+    uint32_t distinct, found; // candidates to test, and their hits
+    __device__ __forceinline__ static void sync() {
+        if constexpr (kWarps == 1u) {
             __syncwarp();
+        } else {
+            __syncthreads();
         }
     }
+    // Bitonic sort of `width` (a power of two) of its values, ascending.
+    template <typename T>
+    __device__ __forceinline__ static void sort(T* values, uint32_t width) {
+#pragma unroll 1
+        for (uint32_t k = 2u; k <= width; k <<= 1) {
+#pragma unroll 1
+            for (uint32_t j = k >> 1; j > 0u; j >>= 1) {
+#pragma unroll 1
+                for (uint32_t index = threadIdx.x % kThreads; index < width; index += kThreads) {
+                    const uint32_t other = index ^ j;
+                    if (other > index) {
+                        const bool ascending = (index & k) == 0u;
+                        const T a = values[index], b = values[other];
+                        if (ascending ? a > b : a < b) {
+                            values[index] = b;
+                            values[other] = a;
+                        }
+                    }
+                }
+                sync();
+            }
+        }
+    }
+};
+// Places for the lanes that ask, from a count the team shares.
+__device__ __forceinline__ uint32_t warp_places(uint32_t* count, bool mine) {
+    const uint32_t mask = __ballot_sync(kFull, mine), lane = threadIdx.x & 31u;
+    uint32_t base = 0u;
+    if (lane == 0u && mask != 0u) base = atomicAdd(count, __popc(mask));
+    return __shfl_sync(kFull, base, 0) + __popc(mask & ((1u << lane) - 1u));
 }
 
-// resolve_hit for a slot per lane (has: this lane holds one). The lanes search for their own closest
+// resolve_lane for a slot per lane (has: this lane holds one). The lanes search for their own closest
 // points; then the whole warp takes the inside probes' penetrations in turn (group_convex_hit), which on
 // one lane, the polytope in its local memory, were most of a sphere query's time.
 __device__ __forceinline__ QHit warp_resolve(const Lanes<32>& L, const DeviceWorld& w, const dyn_query_record& q, bool has, uint32_t slot,
-                                             bool whole, QueryWarpShared& sh) {
+                                             bool whole, QuerySearch& sh) {
     Resolved r{q_no_hit(), false};
     if (has) r = resolve_lane(w, q, collider_shape(w, slot), whole);
     uint32_t inside = __ballot_sync(kFull, r.inside);
@@ -649,238 +647,191 @@ __device__ __forceinline__ QHit warp_resolve(const Lanes<32>& L, const DeviceWor
     return r.hit;
 }
 
-// One warp per query (scene_cast.wgsl:434-533), taken from a shared ticket. A block per query left
-// three of its four warps waiting at barriers for the one that tested hits (7 of 16 cycles per
-// instruction), and tested candidates where they lay among their duplicates (8 of 32 threads per
-// instruction): here the distinct ones are packed first, and a ray's candidates that its box test
-// rules out (ray_meets) are dropped before the sort. A query with more candidates than the warp holds goes to
-// k_scene_query_large.
-__global__ void __launch_bounds__(kQueryThreads) k_scene_query(DeviceWorld w, dyn_query_record* queries, dyn_query_hit_record* hits,
-                                                               uint32_t count, uint32_t* __restrict__ large) {
-    __shared__ QueryWarpShared shared[kQueryThreads / 32u];
-    QueryWarpShared& sh = shared[threadIdx.x >> 5];
+// A query by its team (scene_cast.wgsl:434-533), taken from a shared ticket. Every candidate is kept
+// once: of a collider's entries (one per covered cell) the first in the query's cells. A ray's
+// candidates that its box test rules out (ray_meets) are dropped too; the rest are packed before they
+// are tested, so a warp's lanes all hold one. Warps put a query that keeps more than they hold, or
+// meets more than DYN_QUERY_CANDIDATES entries, or covers more than `wide` cells on `list`; blocks
+// take the list's, or (count > 0) the whole batch. Past DYN_QUERY_CANDIDATES entries the reference
+// tests the ones it met up to there, so a block marks what it would leave out and then keeps it all.
+constexpr uint32_t kOut = 1u << 31;
+static_assert((DYN_ENTRY_INDEX_MASK & kOut) == 0u, "a collider slot leaves the mark's bit free");
+template <uint32_t kWarps>
+__global__ void __launch_bounds__(kQueryThreads, kWarps == 1u ? 3 : 2) k_scene_query(DeviceWorld w, dyn_query_record* queries, dyn_query_hit_record* hits,
+                                                               uint32_t count, uint32_t* __restrict__ list, uint32_t wide) {
+    using Team = QueryTeam<kWarps>;
+    constexpr bool kBlock = kWarps > 1u;
+    constexpr uint32_t kThreads = Team::kThreads;
+    extern __shared__ __align__(16) unsigned char smem[];
+    Team& sh = reinterpret_cast<Team*>(smem)[threadIdx.x / kThreads];
     const Lanes<32> L;
-    const uint32_t lane = L.lane, lane_lt = (1u << lane) - 1u;
+    const uint32_t rank = threadIdx.x % kThreads, warp = rank >> 5;
     const uint32_t live = min(w.ctl[CTL_ENTRIES], w.e_cap);
     const float grid = base_cell(w);
     const uint32_t bits = cell_table_bits(w, live);
     const bool table_overflow = w.ctl[CTL_CELL_OVERFLOW] != 0u;
     const uint32_t levels = w.counters[DYN_COUNTER_GRID_LEVELS] | w.counters[DYN_COUNTER_RESTING_LEVELS] |
                             w.counters[DYN_COUNTER_IMMOVABLE_LEVELS];
+    const bool listed = kBlock && count == 0u;
+    const uint32_t items = listed ? w.ctl[CTL_QUERY_LARGE] : count;
     for (;;) {
-        uint32_t qi = 0u;
-        if (lane == 0u) qi = atomicAdd(&w.ctl[CTL_QUERY_NEXT], 1u);
-        qi = __shfl_sync(kFull, qi, 0);
-        if (qi >= count) break;
+        if (rank == 0u) {
+            sh.next = atomicAdd(&w.ctl[kBlock ? CTL_QUERY_LARGE_NEXT : CTL_QUERY_NEXT], 1u);
+            sh.seen = sh.kept = sh.distinct = sh.found = 0u;
+        }
+        Team::sync();
+        if (sh.next >= items) break;
+        const uint32_t qi = listed ? list[sh.next] : sh.next;
         const dyn_query_record q = queries[qi];
-        if (lane == 0u) sh.seen = sh.kept = 0u;
-        __syncwarp();
         // the candidates: entries of the cells the query's box covers, level by level
         const DAabb box = query_box(w, q);
+        const uint32_t wanted = (q.filters.targets & DYN_QUERY_TARGET_COLLIDERS) != 0u ? levels : 0u;
         const bool is_ray = q.kind == DYN_QUERY_RAY;
         const f3 origin = q_origin(q), heading = is_ray ? normalize(q_direction(q)) : s3(0.0f);
         const bool drops = is_ray && fabsf(dot(heading, heading) - 1.0f) < 1e-3f;
-        auto push = [&](const GEntry& e) {
+        auto cells_of = [&](uint32_t level, float cs, I3* lo, I3* hi) {
+            *lo = floor_div(box.min, cs);
+            *hi = floor_div(box.max, cs);
+            return ((long long)hi->x - lo->x + 1) * ((long long)hi->y - lo->y + 1) * ((long long)hi->z - lo->z + 1);
+        };
+        auto push = [&](const GEntry& e, bool again) {
             const uint32_t seen = atomicAdd(&sh.seen, 1u);
             if (seen >= DYN_QUERY_CANDIDATES) return;
             const uint32_t slot = e.info & DYN_ENTRY_INDEX_MASK;
-            if (drops && !ray_meets(origin, heading, q.extent, e.mn, e.mx) && (w.c_class[slot].w & kClassBoxedRays)) return;
-            const uint32_t at = atomicAdd(&sh.kept, 1u);
-            if (at < kWarpCandidates) sh.candidates[at] = slot;
-        };
-        uint32_t occupied = (q.filters.targets & DYN_QUERY_TARGET_COLLIDERS) != 0u ? levels : 0u;
-#pragma unroll 1
-        while (occupied != 0u) {
-            const uint32_t level = (uint32_t)__ffs(occupied) - 1u;
-            occupied &= occupied - 1u;
-            const float cs = level_size(level, grid);
-            const I3 lo = floor_div(box.min, cs), hi = floor_div(box.max, cs);
-            const long long sx = (long long)hi.x - lo.x + 1, sy = (long long)hi.y - lo.y + 1, sz = (long long)hi.z - lo.z + 1;
-            const long long cells = sx * sy * sz;
-            if (cells <= 0) continue;
-            if (cells > (long long)kGridWalkCells) {
-                // the whole level, its entries tested against the box
-                const uint32_t first = lower_bound(w.ekey, live, level << DYN_LEVEL_KEY_SHIFT);
-                const uint32_t end = lower_bound(w.ekey, live, (level + 1u) << DYN_LEVEL_KEY_SHIFT);
-                for (uint32_t j = first + lane; j < end && sh.seen <= DYN_QUERY_CANDIDATES; j += 32u) {
-                    const GEntry e = load_entry(w, w.eval[j]);
-                    if (!(e.mn.x <= box.max.x && e.mn.y <= box.max.y && e.mn.z <= box.max.z && box.min.x <= e.mx.x &&
-                          box.min.y <= e.mx.y && box.min.z <= e.mx.z))
-                        continue;
-                    push(e);
-                }
+            const bool out = again || (drops && !ray_meets(origin, heading, q.extent, e.mn, e.mx) &&
+                                       (w.c_class[slot].w & kClassBoxedRays));
+            if constexpr (kBlock) {
+                sh.candidates[seen] = slot | (out ? kOut : 0u);
             } else {
-                const uint32_t rows = (uint32_t)(sy * sz);
-                for (uint32_t c = lane; c < (uint32_t)cells; c += 32u) {
-                    const I3 cell = I3{lo.x + (int)(c / rows), lo.y + (int)((c / (uint32_t)sz) % (uint32_t)sy), lo.z + (int)(c % (uint32_t)sz)};
-                    const uint32_t key = cell_key(level, cell);
-                    uint32_t j = cell_find(w, live, bits, table_overflow, key);
-                    if (j >= live) continue;
-                    const uint32_t end = j + __ldg(&w.erun[j].y);
-                    for (; j < end; ++j) push(load_entry(w, w.eval[j]));
+                if (out) return;
+                const uint32_t place = atomicAdd(&sh.kept, 1u);
+                if (place < Team::kCap) sh.candidates[place] = slot;
+            }
+        };
+        bool handed = false;
+        if (!kBlock && wide != 0u) {
+            long long walk = 0;
+            for (uint32_t rest = wanted; rest != 0u; rest &= rest - 1u) {
+                const uint32_t level = (uint32_t)__ffs(rest) - 1u;
+                I3 lo, hi;
+                const long long cells = cells_of(level, level_size(level, grid), &lo, &hi);
+                if (cells > 0) walk += cells;
+                handed = handed || walk > (long long)wide;
+            }
+        }
+        if (!handed) {
+            uint32_t occupied = wanted;
+#pragma unroll 1
+            while (occupied != 0u) {
+                const uint32_t level = (uint32_t)__ffs(occupied) - 1u;
+                occupied &= occupied - 1u;
+                const float cs = level_size(level, grid);
+                I3 lo, hi;
+                const long long cells = cells_of(level, cs, &lo, &hi);
+                if (cells <= 0) continue;
+                if (cells > (long long)kGridWalkCells) {
+                    // the whole level, its entries tested against the box
+                    const uint32_t first = lower_bound(w.ekey, live, level << DYN_LEVEL_KEY_SHIFT);
+                    const uint32_t end = lower_bound(w.ekey, live, (level + 1u) << DYN_LEVEL_KEY_SHIFT);
+                    for (uint32_t j = first + rank; j < end && sh.seen <= DYN_QUERY_CANDIDATES; j += kThreads) {
+                        const GEntry e = load_entry(w, w.eval[j]);
+                        if (!(e.mn.x <= box.max.x && e.mn.y <= box.max.y && e.mn.z <= box.max.z && box.min.x <= e.mx.x &&
+                              box.min.y <= e.mx.y && box.min.z <= e.mx.z))
+                            continue;
+                        push(e, (e.info & DYN_ENTRY_PRIMARY) == 0u);
+                    }
+                } else {
+                    const uint32_t sy = (uint32_t)(hi.y - lo.y + 1), sz = (uint32_t)(hi.z - lo.z + 1), rows = sy * sz;
+                    for (uint32_t c = rank; c < (uint32_t)cells; c += kThreads) {
+                        const I3 cell = I3{lo.x + (int)(c / rows), lo.y + (int)((c / sz) % sy), lo.z + (int)(c % sz)};
+                        const uint32_t key = cell_key(level, cell);
+                        uint32_t j = cell_find(w, live, bits, table_overflow, key);
+                        if (j >= live) continue;
+                        const uint32_t end = j + __ldg(&w.erun[j].y);
+                        for (; j < end; ++j) {
+                            const GEntry e = load_entry(w, w.eval[j]);
+                            push(e, entry_again(e, cs, lo, cell));
+                        }
+                    }
                 }
             }
         }
-        __syncwarp();
-        const uint32_t total = sh.kept;
-        if (total > kWarpCandidates || sh.seen > DYN_QUERY_CANDIDATES) {
-            if (lane == 0u) large[atomicAdd(&w.ctl[CTL_QUERY_LARGE], 1u)] = qi;
-            __syncwarp();
+        Team::sync();
+        uint32_t* packed = reinterpret_cast<uint32_t*>(sh.keys);
+        if constexpr (kBlock) {
+            const uint32_t met = min(sh.seen, DYN_QUERY_CANDIDATES);
+            const bool every = sh.seen > DYN_QUERY_CANDIDATES;
+#pragma unroll 1
+            for (uint32_t base = 0; base < met; base += kThreads) {
+                const uint32_t word = base + rank < met ? sh.candidates[base + rank] : kOut;
+                const bool keep = base + rank < met && (every || (word & kOut) == 0u);
+                const uint32_t place = warp_places(&sh.kept, keep);
+                if (keep) packed[place] = word & ~kOut;
+            }
+            Team::sync();
+            for (uint32_t i = rank; i < sh.kept; i += kThreads) sh.candidates[i] = packed[i];
+            Team::sync();
+        } else if (handed || sh.kept > Team::kCap || sh.seen > DYN_QUERY_CANDIDATES) {
+            __syncwarp();  // every lane has read the counts
+            if (rank == 0u) list[atomicAdd(&w.ctl[CTL_QUERY_LARGE], 1u)] = qi;
             continue;
         }
+        const uint32_t total = sh.kept;
         uint32_t width = 1u;
         while (width < total) width <<= 1;
-        for (uint32_t i = total + lane; i < width; i += 32u) sh.candidates[i] = 0xFFFFFFFFu;
-        __syncwarp();
-        warp_bitonic(sh.candidates, width);
-        // the distinct ones (a collider has an entry per covered cell) that pass the filters, packed
-        uint32_t distinct = 0u;
+        for (uint32_t i = total + rank; i < width; i += kThreads) sh.candidates[i] = 0xFFFFFFFFu;
+        Team::sync();
+        Team::sort(sh.candidates, width);
+        // the distinct ones (cells whose hashes meet give an entry twice) that pass the filters, packed
+        // in the keys' space, since their neighbours are compared with them, then back
 #pragma unroll 1
-        for (uint32_t base = 0; base < total; base += 32u) {
-            const uint32_t i = base + lane;
+        for (uint32_t base = 0; base < total; base += kThreads) {
+            const uint32_t i = base + rank;
             uint32_t slot = 0u;
             bool keep = false;
             if (i < total) {
                 slot = sh.candidates[i];
                 keep = (i == 0u || sh.candidates[i - 1u] != slot) && query_passes(w, q, slot);
             }
-            const uint32_t mask = __ballot_sync(kFull, keep);
-            // the words written lie before the ones later rounds read, except the last word of this
-            // round, which the next compares with: the packed slots go to the keys' space
-            if (keep) reinterpret_cast<uint32_t*>(sh.keys)[kWarpCandidates + distinct + __popc(mask & lane_lt)] = slot;
-            distinct += __popc(mask);
+            const uint32_t place = warp_places(&sh.distinct, keep);
+            if (keep) packed[place] = slot;
         }
-        __syncwarp();
-        for (uint32_t i = lane; i < distinct; i += 32u) sh.candidates[i] = reinterpret_cast<const uint32_t*>(sh.keys)[kWarpCandidates + i];
-        __syncwarp();
-        // their hits, keyed by (distance key, candidate)
-        uint32_t hit_total = 0u;
+        Team::sync();
+        const uint32_t distinct = sh.distinct;
+        for (uint32_t i = rank; i < distinct; i += kThreads) sh.candidates[i] = packed[i];
+        Team::sync();
+        // their hits, keyed by (distance key, candidate); a few candidates are spread over the warps
 #pragma unroll 1
-        for (uint32_t base = 0; base < distinct; base += 32u) {
-            const uint32_t i = base + lane;
+        for (uint32_t base = 0; base < distinct; base += kThreads) {
+            const uint32_t i = base + L.lane * kWarps + warp;
             const bool has = i < distinct;
             const uint32_t slot = has ? sh.candidates[i] : 0u;
-            const QHit hit = warp_resolve(L, w, q, has, slot, false, sh);
+            const QHit hit = warp_resolve(L, w, q, has, slot, false, sh.search[warp]);
             const bool found = hit.distance < kQNoHit;
-            const unsigned long long key = ((unsigned long long)hit_key(hit.distance) << 32) | slot;
-            const uint32_t mask = __ballot_sync(kFull, found);
-            if (found) sh.keys[hit_total + __popc(mask & lane_lt)] = key;
-            hit_total += __popc(mask);
+            const uint32_t place = warp_places(&sh.found, found);
+            if (found) sh.keys[place] = ((unsigned long long)hit_key(hit.distance) << 32) | slot;
         }
+        Team::sync();
+        const uint32_t hit_total = sh.found;
         uint32_t sorted = 1u;
         while (sorted < hit_total) sorted <<= 1;
-        for (uint32_t i = hit_total + lane; i < sorted; i += 32u) sh.keys[i] = ~0ull;
-        __syncwarp();
-        warp_bitonic(sh.keys, sorted);
+        for (uint32_t i = hit_total + rank; i < sorted; i += kThreads) sh.keys[i] = ~0ull;
+        Team::sync();
+        Team::sort(sh.keys, sorted);
         const uint32_t emitted = min(min(q.max_hits, DYN_QUERY_CANDIDATES), hit_total);
 #pragma unroll 1
-        for (uint32_t base = 0; base < emitted; base += 32u) {
-            const uint32_t i = base + lane;
+        for (uint32_t base = 0; base < emitted; base += kThreads) {
+            const uint32_t i = base + L.lane * kWarps + warp;
             const bool has = i < emitted;
             const uint32_t slot = has ? (uint32_t)(sh.keys[i] & 0xFFFFFFFFull) : 0u;
-            const QHit hit = warp_resolve(L, w, q, has, slot, true, sh);
+            const QHit hit = warp_resolve(L, w, q, has, slot, true, sh.search[warp]);
             if (has) write_hit(w, hit, slot, hits + q.hit_base + i);
         }
-        if (lane == 0u) {
+        if (rank == 0u) {
             queries[qi].count = emitted;
-            queries[qi].overflow = emitted < hit_total ? 1u : 0u;
+            queries[qi].overflow = (sh.seen > DYN_QUERY_CANDIDATES || emitted < hit_total) ? 1u : 0u;
         }
-        __syncwarp();
-    }
-}
-
-// One block per query (scene_cast.wgsl:434-533), for the queries with more candidates than a warp holds.
-__global__ void __launch_bounds__(kQueryThreads) k_scene_query_large(DeviceWorld w, dyn_query_record* queries,
-                                                                     dyn_query_hit_record* hits, const uint32_t* __restrict__ list) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    QueryShared& sh = *reinterpret_cast<QueryShared*>(smem);
-    const uint32_t count = w.ctl[CTL_QUERY_LARGE];
-    for (uint32_t at = blockIdx.x; at < count; at += gridDim.x) {
-        const uint32_t qi = list[at];
-        const dyn_query_record q = queries[qi];
-        if (threadIdx.x == 0) {
-            sh.candidate_count = 0u;
-            sh.overflow = 0u;
-            sh.hit_total = 0u;
-        }
-        __syncthreads();
-        // the candidates: entries of the cells the query's box covers, level by level
-        const DAabb box = query_box(w, q);
-        const uint32_t live = min(w.ctl[CTL_ENTRIES], w.e_cap);
-        const float grid = base_cell(w);
-        const uint32_t bits = cell_table_bits(w, live);
-        const bool table_overflow = w.ctl[CTL_CELL_OVERFLOW] != 0u;
-        const bool wants_colliders = (q.filters.targets & DYN_QUERY_TARGET_COLLIDERS) != 0u;
-        uint32_t occupied = wants_colliders ? (w.counters[DYN_COUNTER_GRID_LEVELS] | w.counters[DYN_COUNTER_RESTING_LEVELS] |
-                                                       w.counters[DYN_COUNTER_IMMOVABLE_LEVELS]) : 0u;
-        while (occupied != 0u) {
-            const uint32_t level = (uint32_t)__ffs(occupied) - 1u;
-            occupied &= occupied - 1u;
-            const float cs = level_size(level, grid);
-            const I3 lo = floor_div(box.min, cs), hi = floor_div(box.max, cs);
-            const long long sx = (long long)hi.x - lo.x + 1, sy = (long long)hi.y - lo.y + 1, sz = (long long)hi.z - lo.z + 1;
-            const long long cells = sx * sy * sz;
-            if (cells <= 0) continue;
-            if (cells > (long long)kGridWalkCells) {
-                // the whole level, its entries tested against the box
-                const uint32_t first = lower_bound(w.ekey, live, level << DYN_LEVEL_KEY_SHIFT);
-                const uint32_t end = lower_bound(w.ekey, live, (level + 1u) << DYN_LEVEL_KEY_SHIFT);
-                for (uint32_t j = first + threadIdx.x; j < end && sh.candidate_count <= DYN_QUERY_CANDIDATES; j += blockDim.x) {
-                    const GEntry e = load_entry(w, w.eval[j]);
-                    if (!(e.mn.x <= box.max.x && e.mn.y <= box.max.y && e.mn.z <= box.max.z && box.min.x <= e.mx.x &&
-                          box.min.y <= e.mx.y && box.min.z <= e.mx.z))
-                        continue;
-                    push_candidate(sh, e.info & DYN_ENTRY_INDEX_MASK);
-                }
-            } else {
-                for (uint32_t c = threadIdx.x; c < (uint32_t)cells; c += blockDim.x) {
-                    const uint32_t rows = (uint32_t)(sy * sz);
-                    const I3 cell = I3{lo.x + (int)(c / rows), lo.y + (int)((c / (uint32_t)sz) % (uint32_t)sy), lo.z + (int)(c % (uint32_t)sz)};
-                    const uint32_t key = cell_key(level, cell);
-                    for (uint32_t j = cell_find(w, live, bits, table_overflow, key); j < live && w.ekey[j] == key; ++j) {
-                        const GEntry e = load_entry(w, w.eval[j]);
-                        push_candidate(sh, e.info & DYN_ENTRY_INDEX_MASK);
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        // sorted, duplicates marked (an entry per covered cell of a collider)
-        const uint32_t total = min(sh.candidate_count, DYN_QUERY_CANDIDATES);
-        uint32_t width = 1u;
-        while (width < total) width <<= 1;
-        for (uint32_t i = threadIdx.x; i < width; i += blockDim.x) {
-            if (i >= total) sh.candidates[i] = 0xFFFFFFFFu;
-        }
-        __syncthreads();
-        block_bitonic(sh.candidates, width);
-        // each distinct candidate's hit, keyed by (distance key, candidate)
-        for (uint32_t i = threadIdx.x; i < width; i += blockDim.x) {
-            unsigned long long key = ~0ull;
-            if (i < total && !(i > 0u && sh.candidates[i] == sh.candidates[i - 1u])) {
-                const uint32_t slot = sh.candidates[i];
-                if (query_passes(w, q, slot)) {
-                    const QHit hit = resolve_hit(w, q, collider_shape(w, slot), false);
-                    if (hit.distance < kQNoHit) {
-                        key = ((unsigned long long)hit_key(hit.distance) << 32) | slot;
-                        atomicAdd(&sh.hit_total, 1u);
-                    }
-                }
-            }
-            sh.keys[i] = key;
-        }
-        __syncthreads();
-        block_bitonic(sh.keys, width);
-        const uint32_t emitted = min(min(q.max_hits, DYN_QUERY_CANDIDATES), sh.hit_total);
-        for (uint32_t i = threadIdx.x; i < emitted; i += blockDim.x) {
-            const uint32_t slot = (uint32_t)(sh.keys[i] & 0xFFFFFFFFull);
-            write_hit(w, resolve_hit(w, q, collider_shape(w, slot), true), slot, hits + q.hit_base + i);
-        }
-        if (threadIdx.x == 0) {
-            queries[qi].count = emitted;
-            queries[qi].overflow = (sh.overflow != 0u || emitted < sh.hit_total) ? 1u : 0u;
-        }
-        __syncthreads();
+        Team::sync();
     }
 }
 

@@ -115,6 +115,7 @@ struct DeviceState {
     float4* query_entries = nullptr;
     uint32_t* query_words = nullptr;
     uint32_t query_cap = 0, hit_cap = 0;
+    uint32_t query_count = 0, query_to_blocks = 0;  // the last batch, and how much of it went to blocks at once
     // sort and scan scratch
     uint32_t* op_words = nullptr;  // the operator's and the queries' words (SortWords), cleared by each call
     uint32_t* lookback = nullptr;  // the digit passes' look-back words, cleared by the histogram kernel
@@ -2482,12 +2483,20 @@ DYN_API dyn_status dyn_query(dyn_world* w, dyn_query_record* queries, uint32_t n
     k_cell_clear<<<blocks_for(d, 1u << dw.cell_bits, 256), 256, 0, s>>>(dw);
     k_cell_insert<<<blocks_for(d, E, 256), 256, 0, s>>>(dw);
     DYN_CUDA(cudaMemcpyAsync(d->query_buf, queries, (size_t)n * sizeof(dyn_query_record), cudaMemcpyHostToDevice, s));
-    const size_t smem = sizeof(QueryShared);
-    DYN_CUDA(cudaFuncSetAttribute(k_scene_query_large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_scene_query<<<std::min<uint32_t>(div_up(n, kQueryThreads / 32u), d->sms * 4u), kQueryThreads, 0, s>>>(dw, d->query_buf, d->hit_buf,
-                                                                                                  n, d->query_list);
-    k_scene_query_large<<<std::min<uint32_t>(n, d->sms * 4u), kQueryThreads, smem, s>>>(dw, d->query_buf, d->hit_buf, d->query_list);
+    const size_t warp_smem = 4u * sizeof(QueryTeam<1u>), block_smem = sizeof(QueryTeam<4u>);
+    DYN_CUDA(cudaFuncSetAttribute(k_scene_query<1u>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)warp_smem));
+    DYN_CUDA(cudaFuncSetAttribute(k_scene_query<4u>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem));
+    const uint32_t blocks = std::min<uint32_t>(n, d->sms * 4u);
+    uint32_t to_blocks = n;
+    if (n > d->sms * kBlockQueriesPerSm) {  // a warp each, then a block for those the warps hand on
+        k_scene_query<1u><<<std::min<uint32_t>(div_up(n, 4u), d->sms * 4u), kQueryThreads, warp_smem, s>>>(
+            dw, d->query_buf, d->hit_buf, n, d->query_list, n <= d->sms * kWideQueriesPerSm ? kWideCells : 0u);
+        to_blocks = 0u;
+    }
+    k_scene_query<4u><<<blocks, kQueryThreads, block_smem, s>>>(dw, d->query_buf, d->hit_buf, to_blocks, d->query_list, 0u);
     DYN_CUDA(cudaGetLastError());
+    d->query_count = n;
+    d->query_to_blocks = to_blocks;
     DYN_CUDA(cudaMemcpyAsync(queries, d->query_buf, (size_t)n * sizeof(dyn_query_record), cudaMemcpyDeviceToHost, s));
     if (base) DYN_CUDA(cudaMemcpyAsync(hits, d->hit_buf, (size_t)base * sizeof(dyn_query_hit_record), cudaMemcpyDeviceToHost, s));
     DYN_CUDA(cudaStreamSynchronize(s));
@@ -2506,6 +2515,23 @@ DYN_API dyn_status dyn_hull_triangles(const dyn_world* w, uint32_t source, uint3
 
 // The frozen contacts the next step reads (rest.cuh), six words each: first body id, its
 // generation, second body id, its generation, collider a, collider b; in store order.
+DYN_API dyn_status dyn_debug_paths(dyn_world* w, uint32_t* out) {
+    if (!w || !out || !w->dev) return DYN_ERR_INVALID;
+    DeviceState* d = w->dev;
+    DYN_CUDA(cudaStreamSynchronize(d->stream));
+    uint32_t ctl[CTL_COUNT];
+    DYN_CUDA(cudaMemcpy(ctl, d->dw.ctl, sizeof(ctl), cudaMemcpyDeviceToHost));
+    out[0] = std::min(ctl[CTL_GJK_PAIRS], d->p_cap);
+    out[1] = ctl[CTL_CCD_SWEEPS];
+    out[2] = out[3] = 0u;
+    if (d->query_words) {
+        DYN_CUDA(cudaMemcpy(ctl, d->query_words + 64, sizeof(ctl), cudaMemcpyDeviceToHost));
+        out[3] = d->query_to_blocks ? d->query_to_blocks : ctl[CTL_QUERY_LARGE];
+        out[2] = d->query_count - out[3];
+    }
+    return DYN_OK;
+}
+
 DYN_API dyn_status dyn_debug_resting(dyn_world* w, uint32_t* out, uint32_t cap, uint32_t* count) {
     if (!w || !w->dev) return DYN_ERR_INVALID;
     DeviceState* d = w->dev;

@@ -377,6 +377,12 @@ class World:
         self._check(lib.dyn_debug_islands(self._h, ptr(out), n.value, None))
         return out
 
+    def debug_paths(self) -> dict:
+        """Which kernels the last step's and the last query batch's work went to (dyn_debug_paths)."""
+        out = np.zeros(4, np.uint32)
+        self._check(lib.dyn_debug_paths(self._h, ptr(out)))
+        return dict(zip(("gjk_pairs", "ccd_sweeps", "warp_queries", "block_queries"), out.tolist()))
+
     def query(self, queries: np.ndarray) -> tuple[np.ndarray, np.ndarray]:
         """dyn_query: a batch of scene queries (records.QUERY, e.g. from records.ray_query) against the
         current states. Returns the records (hit_base, count and overflow set) and the hit array

@@ -197,6 +197,10 @@ DYN_API dyn_status dyn_debug_entries(dyn_world* world, uint32_t* keys, uint32_t*
 DYN_API dyn_status dyn_debug_pairs(dyn_world* world, uint32_t* major, uint32_t* minor, uint32_t cap, uint32_t* count);
 DYN_API dyn_status dyn_debug_contacts(dyn_world* world, dyn_contact_record* out, uint32_t cap, uint32_t* count);
 DYN_API dyn_status dyn_debug_islands(dyn_world* world, uint32_t* out, uint32_t cap, uint32_t* count);
+/* Which kernels the work went to (synchronises), four words: the convex pairs the last step's GJK
+ * searched, the directions its continuous collision swept, and of the last dyn_query's batch the
+ * queries a warp answered and those a block did. */
+DYN_API dyn_status dyn_debug_paths(dyn_world* world, uint32_t* out);
 /* Scene queries: World::ray_query, sphere_query, cuboid_query, point_query, overlap_query and
  * sweep_query, then resolve_queries and query_hits (crates/dynamis-world/src/query.rs:50-175;
  * scene_cast.wgsl), as one synchronous call against the world's current body states. Each record

@@ -206,6 +206,7 @@ extern "C" {
     pub fn dyn_debug_pairs(world: *mut DynWorld, major: *mut u32, minor: *mut u32, cap: u32, count: *mut u32) -> DynStatus;
     pub fn dyn_debug_contacts(world: *mut DynWorld, out: *mut ContactRecord, cap: u32, count: *mut u32) -> DynStatus;
     pub fn dyn_debug_islands(world: *mut DynWorld, out: *mut u32, cap: u32, count: *mut u32) -> DynStatus;
+    pub fn dyn_debug_paths(world: *mut DynWorld, out: *mut u32) -> DynStatus;
     pub fn dyn_debug_resting(world: *mut DynWorld, out: *mut u32, cap: u32, count: *mut u32) -> DynStatus;
     pub fn dyn_query(world: *mut DynWorld, queries: *mut QueryRecord, n: u32, hits: *mut QueryHitRecord, hit_capacity: u32) -> DynStatus;
     pub fn dyn_hull_triangles(world: *const DynWorld, source: u32, out: *mut u32, cap: u32, count: *mut u32) -> DynStatus;

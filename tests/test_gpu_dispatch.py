@@ -6,7 +6,8 @@
   just below and above the line give the oracle's pair list.
 * The sorts' tiles hold 4,096 keys, and up to three grid runs share a sort's launches: key counts at
   the tile edges against numpy, and a half-resting world against the oracle.
-* A query with more than 512 candidates leaves its warp for a block.
+* A query batch of up to two an SM goes to blocks, a larger one to warps, which hand on to blocks
+  the queries that keep more than 512 candidates or, up to eight queries an SM, cover many cells.
 * A restored world repeats its steps, its contact stream far from full.
 """
 import numpy as np
@@ -49,6 +50,7 @@ def test_gjk_batches_on_both_sides_of_the_group_line(side):
     world.step(DT)
     oracle.step(DT)
     world.wait()
+    assert (world.debug_paths()["gjk_pairs"] > 8192) == (side == 26)
     compare_step(world, oracle, 0)
     world.close()
 
@@ -110,20 +112,69 @@ def test_three_grid_runs_of_uneven_size_share_a_sort():
     world.close()
 
 
-def test_a_query_with_many_candidates_leaves_its_warp():
+def query_mix(world):
+    """Every kind, from a few candidates to more than a warp holds (none past the limit)."""
+    at = world.read_states()["position"][:-1]
+    centre = np.median(at, axis=0)
+    quat = np.array([0.1, -0.4, 0.2, 0.88])
+    quat /= np.linalg.norm(quat)
+    box, ball = dict(kind=R.SHAPE_CUBOID, half_extents=(1.2, 0.4, 0.8)), dict(kind=R.SHAPE_SPHERE, radius=0.4)
+    all_hits = R.query_filter(max_hits=4096)
+    queries = [R.sphere_query(centre, float(r), all_hits) for r in (0.3, 1.5, 3.0, 3.6)]
+    queries += [R.ray_query((x, 40.0, z), (0.0, -1.0, 0.0), 60.0, R.query_filter(max_hits=64)) for x, _, z in at[::200]]
+    queries += [R.ray_query(centre - (30.0, 0.0, 20.0), (30.0, 0.2, 20.0), 80.0, R.query_filter(max_hits=64))]
+    queries += [R.overlap_query(box, quat, p, R.query_filter(max_hits=32)) for p in at[::400]]
+    queries += [R.overlap_query(dict(kind=R.SHAPE_CUBOID, half_extents=(2.0, 1.5, 2.0)), quat, centre, all_hits)]
+    queries += [R.sweep_query(ball, quat, p + (0.0, 6.0, 0.0), (0.3, -1.0, 0.1), 12.0, R.query_filter(max_hits=8)) for p in at[::500]]
+    queries += [R.point_query(at[7]), R.cuboid_query(at[11], (0.3, 0.3, 0.3))]
+    return queries
+
+
+@pytest.fixture(scope="module")
+def query_world():
     world = World()
     scenes.mixed_pile(14, seed=2).build(world)
     for _ in range(90):
         world.step(DT)
     world.wait()
-    at = world.read_states()["position"][:-1]
-    centre = np.median(at, axis=0)
-    # radii whose boxes hold a few dozen, several hundred and more than 512 entries (all below the 4,096 kept), in one batch
-    compare_queries(world, [R.sphere_query(centre, float(r), R.query_filter(max_hits=4096)) for r in (0.3, 1.5, 3.0, 3.6)] +
-                    [R.ray_query((x, 40.0, z), (0.0, -1.0, 0.0), 60.0, R.query_filter(max_hits=64))
-                     for x, _, z in at[::200]] +
-                    [R.ray_query(centre - (30.0, 0.0, 20.0), (30.0, 0.2, 20.0), 80.0, R.query_filter(max_hits=64))])
+    queries = query_mix(world)
+    small, hits = compare_queries(world, queries)  # against the oracle
+    assert world.debug_paths()["block_queries"] == len(queries)
+    yield world, np.concatenate(queries), small, hits
     world.close()
+
+
+@pytest.mark.parametrize("per_sm", [1, 3, 9])
+def test_query_batches_on_both_sides_of_the_lines(query_world, per_sm):
+    # the same queries again and again, up to per_sm of them an SM: blocks, then warps that hand on the
+    # wide ones, then warps that hand on only what they cannot hold
+    world, mix, small, hits = query_world
+    n = per_sm * torch.cuda.get_device_properties(0).multi_processor_count
+    pick = np.arange(n) % len(mix)
+    got, got_hits = world.query(mix[pick])
+    paths = world.debug_paths()
+    if per_sm == 1:
+        assert paths["warp_queries"] == 0
+    elif per_sm == 3:
+        assert 0 < paths["warp_queries"] < n // 2
+    else:
+        assert n // 2 < paths["warp_queries"] < n
+    for name in ("count", "overflow"):
+        assert np.array_equal(got[name], small[name][pick]), name
+    for i, j in enumerate(pick):
+        one = got_hits[got["hit_base"][i]: got["hit_base"][i] + got["count"][i]]
+        want = hits[small["hit_base"][j]: small["hit_base"][j] + small["count"][j]]
+        assert one.tobytes() == want.tobytes(), f"query {i}"
+
+
+@pytest.mark.parametrize("copies", [1, 500])
+def test_a_query_past_the_candidate_limit_is_flagged(query_world, copies):
+    # a box over most of the pile meets more than the 4,096 entries a query takes
+    world, mix = query_world[0], query_world[1]
+    centre = mix["origin"][0]
+    got, _ = world.query(np.concatenate([R.sphere_query(centre, 6.0, R.query_filter(max_hits=8))] * copies))
+    assert np.all(got["overflow"] == 1) and np.all(got["count"] == 8)
+    assert world.debug_paths()["block_queries"] == copies
 
 
 def test_a_restored_world_repeats_its_steps_with_most_of_the_stream_empty():
