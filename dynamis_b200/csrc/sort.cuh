@@ -5,7 +5,7 @@
 // the minor word's digits first and then the major word's (radix.rs:312-317), a u32 payload
 // carried along. Design is new:
 //   * one up-front histogram kernel counts every digit pass in a single read of the keys;
-//   * each digit pass is ONE kernel: a tile of 512 threads x 8 keys ranks its keys with
+//   * each digit pass is ONE kernel: a tile of 512 or 256 threads x 8 keys ranks its keys with
 //     warp __match_any_sync (stable: rounds in index order, lanes in order), publishes its digit
 //     counts, and resolves its global digit prefix by decoupled look-back over earlier tiles;
 //   * up to three arrays are sorted apart by the same launches (SortSource's segments);
@@ -22,9 +22,19 @@
 
 namespace dyn {
 
-constexpr int kSortThreads = 512;
 constexpr int kSortItems = 8;
-constexpr int kSortTile = kSortThreads * kSortItems;  // 4096 keys
+// Tiles: 512 threads (4096 keys), or 256 (2048) while every such tile has an SM of its own. A tile's
+// time is its chain of eight ranking rounds, whose match instructions share the SM's four schedulers,
+// so half the warps finish it sooner; past that the wide tile's fewer look-backs win. Two words with a
+// payload, three digits each, us a sort, wide / narrow: 4,096 keys 80 / 56, 30,000 82 / 68, 130,000
+// 97 / 76, 300,000 99 / 86, 500,000 103 / 111.
+constexpr uint32_t kSortWide = 512u, kSortNarrow = 256u;
+constexpr uint32_t kSortNarrowKeys = 148u * kSortNarrow * kSortItems;
+__host__ __device__ __forceinline__ uint32_t sort_threads(uint32_t cap) { return cap <= kSortNarrowKeys ? kSortNarrow : kSortWide; }
+__host__ __device__ __forceinline__ uint32_t sort_tiles(uint32_t keys, uint32_t threads) {
+    const uint32_t tile = threads * kSortItems;
+    return (keys + tile - 1u) / tile;
+}
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;  // 2048 values
@@ -55,18 +65,18 @@ __device__ __forceinline__ uint32_t sort_count(const SortSource& s, uint32_t seg
     return s.count[segment] ? min(*s.count[segment], s.cap) : s.n_fixed;
 }
 // Tickets in flight at most (one per tile) for segments whose keys together fit `cap`.
-__host__ __device__ __forceinline__ uint32_t sort_tickets(uint32_t cap, uint32_t segments) {
-    return (cap + kSortTile - 1) / kSortTile + segments - 1u + (cap == 0u ? 1u : 0u);
+__host__ __device__ __forceinline__ uint32_t sort_tickets(uint32_t cap, uint32_t segments, uint32_t threads) {
+    return sort_tiles(cap, threads) + segments - 1u + (cap == 0u ? 1u : 0u);
 }
 // The tile a ticket stands for: its segment, the segment's first ticket, its keys.
 struct SortTilePlace {
     uint32_t segment, first_ticket, n, packed;  // packed: the segment's first word in the alternate buffers
     bool live;
 };
-__device__ __forceinline__ SortTilePlace sort_place(const SortSource& s, uint32_t ticket) {
+__device__ __forceinline__ SortTilePlace sort_place(const SortSource& s, uint32_t ticket, uint32_t threads) {
     SortTilePlace t{0u, 0u, 0u, 0u, false};
     for (uint32_t segment = 0; segment < s.segments; ++segment) {
-        const uint32_t n = sort_count(s, segment), tiles = (n + kSortTile - 1) / kSortTile;
+        const uint32_t n = sort_count(s, segment), tiles = sort_tiles(n, threads);
         if (ticket < t.first_ticket + tiles) {
             t.segment = segment;
             t.n = n;
@@ -81,17 +91,17 @@ __device__ __forceinline__ SortTilePlace sort_place(const SortSource& s, uint32_
 
 // Counts digit occurrences for every pass of the sort in one read, and clears the look-back words of
 // the tiles its passes will run. hist: segments x passes x 256 words; lookback: passes x tickets x
-// 256 words. Digit pass p reads word (p < minor_digits ? minor : major), byte (p or p - minor_digits).
+// 256 words; `threads`: a pass's. Digit pass p reads word (p < minor_digits ? minor : major), byte (p or p - minor_digits).
 static __global__ void k_sort_histogram(const uint32_t* __restrict__ major, const uint32_t* __restrict__ minor, SortSource src,
                                         int major_digits, int minor_digits, uint32_t* __restrict__ hist,
-                                        uint32_t* __restrict__ lookback, uint32_t tickets) {
+                                        uint32_t* __restrict__ lookback, uint32_t tickets, uint32_t threads) {
     __shared__ uint32_t local[8][256];
     const int passes = major_digits + minor_digits;
     uint32_t tiles = 0u;
     for (uint32_t segment = 0; segment < src.segments; ++segment) {
         const uint32_t n = sort_count(src, segment);
         if (n == 0u) continue;
-        tiles += (n + kSortTile - 1) / kSortTile;
+        tiles += sort_tiles(n, threads);
         if (blockIdx.x * blockDim.x >= n) continue;
         for (int i = threadIdx.x; i < passes * 256; i += blockDim.x) (&local[0][0])[i] = 0;
         __syncthreads();
@@ -155,29 +165,30 @@ __device__ __forceinline__ void scan_256(uint32_t a, uint32_t b, uint32_t* ea, u
 // its own, a thread looks back over eight tiles' words at a time, and the three arrays leave through
 // one staging buffer in turn, which keeps two blocks on an SM. 1M keys of two words with a payload, six
 // passes and the histogram: 116 -> 94 us.
-template <bool kTwoWords, bool kPayload>
-static __global__ void __launch_bounds__(kSortThreads, 2)
+template <bool kTwoWords, bool kPayload, uint32_t kThreads>
+static __global__ void __launch_bounds__(kThreads, 1024 / kThreads)
     k_onesweep(const uint32_t* __restrict__ key_in, const uint32_t* __restrict__ other_in,
                const uint32_t* __restrict__ val_in, uint32_t* __restrict__ key_out, uint32_t* __restrict__ other_out,
                uint32_t* __restrict__ val_out, SortSource src, bool from_primary, int shift,
                const uint32_t* __restrict__ digit_totals, uint32_t passes, uint32_t* __restrict__ lookback,
                uint32_t* __restrict__ tile_counter, uint32_t* __restrict__ status, uint32_t spin_limit) {
-    constexpr int kWarps = kSortThreads / 32;
+    constexpr int kWarps = kThreads / 32;
+    constexpr uint32_t kTile = kThreads * kSortItems;
     __shared__ uint32_t warp_hist[kWarps][256];
     __shared__ uint32_t tile_start[256];
     __shared__ uint32_t global_start[256];
-    __shared__ uint32_t stage[kSortTile];
+    __shared__ uint32_t stage[kTile];
     __shared__ uint32_t sums[2][8];
     __shared__ uint32_t tile_id;
 
     if (threadIdx.x == 0) tile_id = atomicAdd(tile_counter, 1u);
-    for (int i = threadIdx.x; i < kWarps * 256; i += kSortThreads) (&warp_hist[0][0])[i] = 0u;
+    for (int i = threadIdx.x; i < kWarps * 256; i += kThreads) (&warp_hist[0][0])[i] = 0u;
     __syncthreads();
     const uint32_t ticket = tile_id;
-    const SortTilePlace at = sort_place(src, ticket);
+    const SortTilePlace at = sort_place(src, ticket, kThreads);
     if (!at.live) return;
-    const uint32_t tile_base = (ticket - at.first_ticket) * kSortTile;
-    const uint32_t tile_n = min((uint32_t)kSortTile, at.n - tile_base);
+    const uint32_t tile_base = (ticket - at.first_ticket) * kTile;
+    const uint32_t tile_n = min(kTile, at.n - tile_base);
     const size_t primary = (size_t)at.segment * src.stride;
     const size_t in = (from_primary ? primary : (size_t)at.packed) + tile_base, out = from_primary ? (size_t)at.packed : primary;
     const int warp = threadIdx.x >> 5;
@@ -277,7 +288,7 @@ static __global__ void __launch_bounds__(kSortThreads, 2)
     uint32_t dst[kSortItems];
 #pragma unroll
     for (int r = 0; r < kSortItems; ++r) {
-        const uint32_t i = threadIdx.x + r * kSortThreads;
+        const uint32_t i = threadIdx.x + r * kThreads;
         if (i < tile_n) {
             const uint32_t k = stage[i];
             dst[r] = global_start[(k >> shift) & 255u] + i;
@@ -294,12 +305,23 @@ static __global__ void __launch_bounds__(kSortThreads, 2)
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < kSortItems; ++r) {
-            const uint32_t i = threadIdx.x + r * kSortThreads;
+            const uint32_t i = threadIdx.x + r * kThreads;
             if (i < tile_n && dst[r] < at.n) to[out + dst[r]] = stage[i];
         }
     };
     if (kTwoWords) ride(others, other_out);
     if (kPayload) ride(vals, val_out);
+}
+
+using SortPass = void (*)(const uint32_t*, const uint32_t*, const uint32_t*, uint32_t*, uint32_t*, uint32_t*, SortSource, bool, int,
+                          const uint32_t*, uint32_t, uint32_t*, uint32_t*, uint32_t*, uint32_t);
+template <uint32_t kThreads>
+static SortPass sort_pass(bool two, bool payload) {
+    return two && payload ? k_onesweep<true, true, kThreads> : two ? k_onesweep<true, false, kThreads>
+           : payload ? k_onesweep<false, true, kThreads> : k_onesweep<false, false, kThreads>;
+}
+static inline SortPass sort_pass(bool two, bool payload, uint32_t threads) {
+    return threads == kSortNarrow ? sort_pass<kSortNarrow>(two, payload) : sort_pass<kSortWide>(two, payload);
 }
 
 // Single-pass exclusive scan of u32 values (decoupled look-back over 2048-value tiles).

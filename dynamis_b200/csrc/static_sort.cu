@@ -37,7 +37,8 @@ using namespace dyn;
 
 constexpr uint32_t kMaxKeys = DYN_STATIC_SORT_MAX_KEYS;
 constexpr uint32_t kMaxPasses = 8;
-constexpr uint32_t kMaxTiles = (kMaxKeys + kSortTile - 1) / kSortTile;
+static_assert(kMaxKeys <= kSortNarrowKeys, "every call's tiles are narrow ones");
+constexpr uint32_t kMaxTiles = (kMaxKeys + kSortNarrow * kSortItems - 1) / (kSortNarrow * kSortItems);
 // word offsets inside the scratch array
 constexpr size_t kAltMajor = 0;
 constexpr size_t kAltMinor = kAltMajor + kMaxKeys;
@@ -121,7 +122,7 @@ extern "C" DYN_API dyn_status dyn_radix_sort_static(uint32_t* major, uint32_t* m
         }
     }
     cudaStream_t s = static_cast<cudaStream_t>(cuda_stream);
-    uint32_t tiles = div_up(n, kSortTile);
+    const uint32_t threads = sort_threads(n), tiles = sort_tiles(n, threads);
     uint32_t* hist = scratch + kHist;
     uint32_t* tickets = scratch + kTickets;
     uint32_t* status = scratch + kStatus;
@@ -139,7 +140,7 @@ extern "C" DYN_API dyn_status dyn_radix_sort_static(uint32_t* major, uint32_t* m
     }
     const SortSource src{{nullptr, nullptr, nullptr}, 1u, n, n, 0u};
     k_sort_histogram<<<div_up(n, 256) < 592u ? div_up(n, 256) : 592u, 256, 0, s>>>(major, minor, src, (int)major_digits,
-                                                                                     (int)minor_digits, hist, lookback, tiles);
+                                                                                     (int)minor_digits, hist, lookback, tiles, threads);
     if (cudaGetLastError() != cudaSuccess) return DYN_ERR_CUDA;
     uint32_t* src_major = major;
     uint32_t* src_minor = minor;
@@ -156,9 +157,8 @@ extern "C" DYN_API dyn_status dyn_radix_sort_static(uint32_t* major, uint32_t* m
         uint32_t* oth_in = on_minor ? src_major : src_minor;
         uint32_t* oth_out = on_minor ? dst_major : dst_minor;
         uint32_t* lb = lookback + (size_t)p * tiles * 256;
-        auto pass = two && payload ? k_onesweep<true, true> : two ? k_onesweep<true, false>
-                    : payload ? k_onesweep<false, true> : k_onesweep<false, false>;
-        pass<<<tiles, kSortThreads, 0, s>>>(key_in, oth_in, src_val, key_out, oth_out, dst_val, src, p % 2 == 0, shift,
+        const SortPass pass = sort_pass(two, payload != nullptr, threads);
+        pass<<<tiles, threads, 0, s>>>(key_in, oth_in, src_val, key_out, oth_out, dst_val, src, p % 2 == 0, shift,
                                             hist + p * 256, passes, lb, tickets + p, status, limit);
         if (cudaGetLastError() != cudaSuccess) return DYN_ERR_CUDA;
         uint32_t* t;

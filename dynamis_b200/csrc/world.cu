@@ -190,8 +190,12 @@ constexpr uint32_t kEntryHist = 0u, kContactHist = kMaxSegments * 4u * 256u, kSt
 constexpr uint32_t kStepScans = kStepTickets + 32u;
 constexpr uint32_t kOpTickets = 8u * 256u, kOpScan = kOpTickets + 16u;
 uint32_t scan_words(uint32_t cap) { return 1u + std::max((cap + kScanTile - 1u) / kScanTile, 1u); }
-// Look-back words for the longest sort: eight passes over the entries' segments or the pairs.
-size_t lookback_words(size_t keys) { return (size_t)8 * ((keys + kSortTile - 1) / kSortTile + kMaxSegments) * 256; }
+// Look-back words for the longest sort: eight passes over the entries' segments or the pairs
+// (of the narrow tiles too, while they are used).
+size_t lookback_words(uint32_t keys) {
+    const uint32_t tiles = std::max(sort_tiles(keys, kSortWide), sort_tiles(std::min(keys, kSortNarrowKeys), kSortNarrow));
+    return (size_t)8 * (tiles + kMaxSegments) * 256;
+}
 
 dyn_status alloc_contacts(dyn_world* w, DeviceState* d, ContactSet* s, uint32_t cap) {
     dyn_status st;
@@ -648,9 +652,9 @@ void record_sort(DeviceState* d, cudaStream_t s, uint32_t* major, uint32_t* mino
                  uint32_t minor_digits, uint32_t* hist, uint32_t* tickets, uint32_t spin_limit = kLookbackSpinLimit) {
     uint32_t passes = major_digits + minor_digits;
     if (passes == 0) return;
-    const uint32_t tiles = sort_tickets(cap, src.segments);
+    const uint32_t threads = sort_threads(cap), tiles = sort_tickets(cap, src.segments, threads);
     k_sort_histogram<<<std::min(div_up(cap, 256), d->sms * 4u), 256, 0, s>>>(major, minor, src, (int)major_digits,
-                                                                            (int)minor_digits, hist, d->lookback, tiles);
+                                                                            (int)minor_digits, hist, d->lookback, tiles, threads);
     uint32_t* src_major = major;
     uint32_t* src_minor = minor;
     uint32_t* src_val = val;
@@ -658,8 +662,7 @@ void record_sort(DeviceState* d, cudaStream_t s, uint32_t* major, uint32_t* mino
     uint32_t* dst_minor = minor_alt;
     uint32_t* dst_val = val_alt;
     bool two = minor != nullptr;
-    auto pass = two && val ? k_onesweep<true, true> : two ? k_onesweep<true, false>
-                : val ? k_onesweep<false, true> : k_onesweep<false, false>;
+    const SortPass pass = sort_pass(two, val != nullptr, threads);
     for (uint32_t p = 0; p < passes; ++p) {
         bool on_minor = p < minor_digits;
         int shift = 8 * (int)(on_minor ? p : p - minor_digits);
@@ -667,7 +670,7 @@ void record_sort(DeviceState* d, cudaStream_t s, uint32_t* major, uint32_t* mino
         uint32_t* key_out = on_minor ? dst_minor : dst_major;
         uint32_t* oth_in = on_minor ? src_major : src_minor;
         uint32_t* oth_out = on_minor ? dst_major : dst_minor;
-        pass<<<tiles, kSortThreads, 0, s>>>(key_in, oth_in, src_val, key_out, oth_out, dst_val, src, p % 2 == 0, shift,
+        pass<<<tiles, threads, 0, s>>>(key_in, oth_in, src_val, key_out, oth_out, dst_val, src, p % 2 == 0, shift,
                                             hist + p * 256, passes, d->lookback + (size_t)p * tiles * 256, tickets + p,
                                             d->dw.ctl + CTL_STATUS, spin_limit);
         std::swap(src_major, dst_major);
@@ -1331,7 +1334,7 @@ dyn_status widen_pair_stream(dyn_world* w) {
                      {reinterpret_cast<void**>(&dw.cmin_alt), P * sizeof(uint32_t), nullptr},
                      {reinterpret_cast<void**>(&dw.cval_alt), P * sizeof(uint32_t), nullptr},
                      {reinterpret_cast<void**>(&d->lookback),
-                      lookback_words(std::max<size_t>(d->e_cap, P)) * sizeof(uint32_t), nullptr}};
+                      lookback_words(std::max(d->e_cap, (uint32_t)P)) * sizeof(uint32_t), nullptr}};
     for (Buffer& b : list) {
         if (cudaMalloc(&b.fresh, b.bytes) != cudaSuccess) {
             for (Buffer& f : list) if (f.fresh) cudaFree(f.fresh);

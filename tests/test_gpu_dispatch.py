@@ -4,8 +4,9 @@
   sides of the line are compared with the oracle, contact for contact.
 * The coarse pair walk gives a thread one cell up to 8,192 colliders and a level slice above: fields
   just below and above the line give the oracle's pair list.
-* The sorts' tiles hold 4,096 keys, and up to three grid runs share a sort's launches: key counts at
-  the tile edges against numpy, and a half-resting world against the oracle.
+* The sorts' tiles hold 2,048 keys up to 303,104 and 4,096 above, and up to three grid runs share a
+  sort's launches: key counts at the tile edges and on both sides of the line against numpy, and a
+  half-resting world against the oracle.
 * A query batch of up to two an SM goes to blocks, a larger one to warps, which hand on to blocks
   the queries that keep more than 512 candidates or, up to eight queries an SM, cover many cells.
 * A restored world repeats its steps, its contact stream far from full.
@@ -73,13 +74,14 @@ def test_coarse_walk_on_both_sides_of_the_split(side):
     world.close()
 
 
-@pytest.mark.parametrize("n", [4095, 4096, 4097, 8191, 8192, 8193, 3 * 4096 + 1])
+@pytest.mark.parametrize("n", [2047, 2048, 2049, 4095, 4096, 4097, 8191, 8192, 8193, 3 * 4096 + 1, 148 * 2048, 148 * 2048 + 1,
+                               80 * 4096, 80 * 4096 + 1])
 @pytest.mark.parametrize("words", [1, 2])
 def test_sort_at_the_tile_edges(n, words):
     rng = np.random.default_rng(n + words)
     # few distinct keys, so that the order of equal ones shows
     keys = rng.integers(0, 700, (words, n), dtype=np.int64).astype(np.int32)
-    world = World(capacity={"pairs": 1 << 16})
+    world = World(capacity={"pairs": 1 << 19})
     tensors = [torch.from_numpy(k.copy()).cuda() for k in keys]
     payload = torch.arange(n, dtype=torch.int32, device="cuda")
     torch.cuda.synchronize()

@@ -122,7 +122,8 @@ def test_known_answers_of_the_reference_sort_tests(world):
     assert digest(pay) == wide["payload_sha256"]
 
 
-def test_a_lookback_wait_that_runs_out_is_reported_and_cleared(world):
+@pytest.mark.parametrize("tiles,tile", [(6, 2048), (13, 2048), (83, 4096)])
+def test_a_lookback_wait_that_runs_out_is_reported_and_cleared(world, tiles, tile):
     """The bounded look-back wait, made to run out on purpose: the first tile of every digit pass is
     never run (its ticket is skipped), so the later tiles poll for a word nothing writes until their
     limit of 1,000 polls is spent. Every write stays within the n keys. dyn_sync must then report
@@ -131,7 +132,7 @@ def test_a_lookback_wait_that_runs_out_is_reported_and_cleared(world):
     from dynamis_b200._native import DynamisError
 
     rng = np.random.default_rng(5)
-    n = 5 * 2048 + 17  # six tiles: five of them wait on the missing first one
+    n = (tiles - 1) * tile + 17  # all but one wait on the missing first one, eight tiles at a time
     keys = rng.integers(0, 1 << 30, size=n, dtype=np.uint32)
     check(lib.dyn_debug_sort_fault(world._h, 1, 1000), world._h)
     tm = torch.from_numpy(keys.view(np.int32)).to("cuda:0")

@@ -122,7 +122,7 @@ def test_the_status_of_a_call_is_readable_after_it():
     import ctypes
 
     rng = np.random.default_rng(23)
-    n = 4 * 2048 + 5
+    n = 12 * 2048 + 5  # thirteen tiles: some waits cover a full window of eight
     keys = rng.integers(0, 1 << 32, size=n, dtype=np.uint64).astype(np.uint32)
     stream = torch.cuda.current_stream()
     status = ctypes.c_uint32(7)
