@@ -520,18 +520,23 @@ __device__ __forceinline__ void write_hit(const DeviceWorld& w, const QHit& hit,
 }
 
 // Is this entry, met in `cell`, a repeat of a collider whose entry in an earlier one of the query's
-// cells (from `lo`) is met too? A collider's entries are the cells of its box, two an axis at most; the
-// offset bits tell the lowest from the second. An entry met in another cell than its own (their hashes
-// meet) is no repeat, nor is any of a box that spans more (its coordinates are not finite).
-__device__ __forceinline__ bool entry_again(const GEntry& e, float cs, I3 lo, I3 cell) {
+// cells (from `lo`) is met too? A collider's entries are the cells of its box, two an axis at most
+// below the last level; the offset bits tell the lowest from the second, and the first that the query
+// meets has no bit set but where its cell is the query's lowest. That one is met when the box's cells
+// and the query's share one, as they do when the boxes overlap (floor and division are monotone); an
+// entry met through another cell's hash may share none, and one whose box stays clear is left to the
+// sort.
+__device__ __forceinline__ bool box_overlaps(const GEntry& e, const DAabb& box) {
+    return e.mn.x <= box.max.x && e.mn.y <= box.max.y && e.mn.z <= box.max.z && box.min.x <= e.mx.x && box.min.y <= e.mx.y &&
+           box.min.z <= e.mx.z;
+}
+__device__ __forceinline__ bool entry_again(const GEntry& e, uint32_t level, I3 lo, I3 cell, const DAabb& box) {
     const uint32_t bits = (e.info & DYN_ENTRY_CELL_MASK) >> DYN_ENTRY_CELL_SHIFT;
-    if (!(((bits & 1u) && cell.x != lo.x) || ((bits & 2u) && cell.y != lo.y) || ((bits & 4u) && cell.z != lo.z))) return false;
-    const I3 a = floor_div(e.mn, cs), b = floor_div(e.mx, cs);
-    if ((long long)b.x - a.x > 1 || (long long)b.y - a.y > 1 || (long long)b.z - a.z > 1) return false;
-    return same_cell(I3{a.x + (int)(bits & 1u), a.y + (int)((bits >> 1) & 1u), a.z + (int)((bits >> 2) & 1u)}, cell);
+    const bool later = ((bits & 1u) && cell.x != lo.x) || ((bits & 2u) && cell.y != lo.y) || ((bits & 4u) && cell.z != lo.z);
+    return later && level < DYN_GRID_LEVEL_LIMIT && box_overlaps(e, box);
 }
 
-// Can a ray reach the box at all? Asked for the colliders whose class record says kClassBoxedRays only
+// Can a ray reach the box at all? Asked for the colliders whose entries say kEntryBoxedRays only
 // (unscaled spheres, cuboids, capsules and cylinders); the others always go on to their test: a
 // scaled frame's test answers hits past the ray's end, and a triangle's is unbounded near its plane.
 // For the four, with u = 2^-24 and a unit heading, a test that answers a hit at t has its point o + t d
@@ -656,8 +661,10 @@ __device__ __forceinline__ QHit warp_resolve(const Lanes<32>& L, const DeviceWor
 // tests the ones it met up to there, so a block marks what it would leave out and then keeps it all.
 constexpr uint32_t kOut = 1u << 31;
 static_assert((DYN_ENTRY_INDEX_MASK & kOut) == 0u, "a collider slot leaves the mark's bit free");
+// Warps are held to 128 registers for four blocks an SM (16,384 rays and balls: 7.08 ms against 7.22
+// with three); blocks keep two and their spills out (64 rays of 60 m 1.39 against 1.83 ms with three).
 template <uint32_t kWarps>
-__global__ void __launch_bounds__(kQueryThreads, kWarps == 1u ? 3 : 2) k_scene_query(DeviceWorld w, dyn_query_record* queries, dyn_query_hit_record* hits,
+__global__ void __launch_bounds__(kQueryThreads, kWarps == 1u ? 4 : 2) k_scene_query(DeviceWorld w, dyn_query_record* queries, dyn_query_hit_record* hits,
                                                                uint32_t count, uint32_t* __restrict__ list, uint32_t wide) {
     using Team = QueryTeam<kWarps>;
     constexpr bool kBlock = kWarps > 1u;
@@ -698,8 +705,7 @@ __global__ void __launch_bounds__(kQueryThreads, kWarps == 1u ? 3 : 2) k_scene_q
             const uint32_t seen = atomicAdd(&sh.seen, 1u);
             if (seen >= DYN_QUERY_CANDIDATES) return;
             const uint32_t slot = e.info & DYN_ENTRY_INDEX_MASK;
-            const bool out = again || (drops && !ray_meets(origin, heading, q.extent, e.mn, e.mx) &&
-                                       (w.c_class[slot].w & kClassBoxedRays));
+            const bool out = again || (drops && (e.info & kEntryBoxedRays) && !ray_meets(origin, heading, q.extent, e.mn, e.mx));
             if constexpr (kBlock) {
                 sh.candidates[seen] = slot | (out ? kOut : 0u);
             } else {
@@ -735,9 +741,7 @@ __global__ void __launch_bounds__(kQueryThreads, kWarps == 1u ? 3 : 2) k_scene_q
                     const uint32_t end = lower_bound(w.ekey, live, (level + 1u) << DYN_LEVEL_KEY_SHIFT);
                     for (uint32_t j = first + rank; j < end && sh.seen <= DYN_QUERY_CANDIDATES; j += kThreads) {
                         const GEntry e = load_entry(w, w.eval[j]);
-                        if (!(e.mn.x <= box.max.x && e.mn.y <= box.max.y && e.mn.z <= box.max.z && box.min.x <= e.mx.x &&
-                              box.min.y <= e.mx.y && box.min.z <= e.mx.z))
-                            continue;
+                        if (!box_overlaps(e, box)) continue;
                         push(e, (e.info & DYN_ENTRY_PRIMARY) == 0u);
                     }
                 } else {
@@ -750,7 +754,7 @@ __global__ void __launch_bounds__(kQueryThreads, kWarps == 1u ? 3 : 2) k_scene_q
                         const uint32_t end = j + __ldg(&w.erun[j].y);
                         for (; j < end; ++j) {
                             const GEntry e = load_entry(w, w.eval[j]);
-                            push(e, entry_again(e, cs, lo, cell));
+                            push(e, entry_again(e, level, lo, cell, box));
                         }
                     }
                 }

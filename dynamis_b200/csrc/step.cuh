@@ -228,6 +228,9 @@ __device__ __forceinline__ float grid_extent_of(f3 mn, f3 mx) { return wmax(wmax
 // caller adds "unscaled": a scaled frame's ray test measures the extent in that frame's lengths and
 // answers hits past the ray's end.
 constexpr uint32_t kClassBoxedRays = 0x400u;  // in c_class[].w
+// The same in a query's own entries, which nothing asks whether they are awake: a ray's walk drops most
+// of what it meets, and a load of the class record for each of these took 8 % of a ray batch's time.
+constexpr uint32_t kEntryBoxedRays = DYN_ENTRY_AWAKE;
 __device__ __forceinline__ bool rays_stay_in_box(const WShape& s) {
     const float4 q = s.rotation;
     const float square = q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w;
@@ -439,7 +442,8 @@ __global__ void k_grid_gate(DeviceWorld w) {
 // collider_emit.wgsl:31-63 for the colliders whose entries this launch writes, in collider order at
 // their scanned key positions. A step writes the awake run and every kept run the gate marked
 // stale, each entry into its collider's own slots (8 * collider + ordinal), and records which kept
-// run a collider's slots now hold. A query writes every collider's entries compactly.
+// run a collider's slots now hold. A query writes every collider's entries compactly, with
+// kEntryBoxedRays in place of the awake bit.
 template <bool kStep>
 __global__ void k_entry_emit(DeviceWorld w) {
     float base = base_cell(w);
@@ -479,6 +483,7 @@ __global__ void k_entry_emit(DeviceWorld w) {
         bool mv = moves(h.pos.w, h.aux.y);
         bool awake = w.activity[owner] != 0u || w.wake_flags[owner] != 0u;
         const uint32_t world = w.body_world[owner];
+        const bool boxed = !kStep && (w.c_class[i].w & kClassBoxedRays) != 0u;
         for (uint32_t ordinal = 0; ordinal < emitted; ++ordinal) {
             I3 c = I3{lo.x + (int)(ordinal / rows), lo.y + (int)((ordinal / sz) % sy), lo.z + (int)(ordinal % sz)};
             uint32_t offset = (uint32_t)(c.x - lo.x) | ((uint32_t)(c.y - lo.y) << 1) | ((uint32_t)(c.z - lo.z) << 2);
@@ -486,7 +491,8 @@ __global__ void k_entry_emit(DeviceWorld w) {
             keys[first + ordinal] = cell_key_in(level, c, world);
             vals[first + ordinal] = slot;
             w.entries[2 * slot] = make_float4(mn.x, mn.y, mn.z, __uint_as_float(owner));
-            w.entries[2 * slot + 1] = make_float4(mx.x, mx.y, mx.z, __uint_as_float(entry_info(i, offset, mv, awake)));
+            const uint32_t info = entry_info(i, offset, mv, kStep && awake) | (boxed ? kEntryBoxedRays : 0u);
+            w.entries[2 * slot + 1] = make_float4(mx.x, mx.y, mx.z, __uint_as_float(info));
         }
     }
 }

@@ -2464,8 +2464,11 @@ DYN_API dyn_status dyn_query(dyn_world* w, dyn_query_record* queries, uint32_t n
     DeviceWorld dw = d->dw;
     const uint32_t K = std::max(dw.k, 1u), E = dw.e_cap;
     cudaStream_t s = d->stream;
+    constexpr size_t warp_smem = 4u * sizeof(QueryTeam<1u>), block_smem = sizeof(QueryTeam<4u>);
     if (!d->query_entries) {
         DYN_CUDA(cudaStreamSynchronize(s));
+        DYN_CUDA(cudaFuncSetAttribute(k_scene_query<1u>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)warp_smem));
+        DYN_CUDA(cudaFuncSetAttribute(k_scene_query<4u>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem));
         DYN_CUDA(cudaMalloc(&d->query_entries, 2 * (size_t)E * sizeof(float4)));
         DYN_CUDA(cudaMalloc(&d->query_words, (64 + CTL_COUNT) * sizeof(uint32_t)));
     }
@@ -2486,10 +2489,7 @@ DYN_API dyn_status dyn_query(dyn_world* w, dyn_query_record* queries, uint32_t n
     k_cell_clear<<<blocks_for(d, 1u << dw.cell_bits, 256), 256, 0, s>>>(dw);
     k_cell_insert<<<blocks_for(d, E, 256), 256, 0, s>>>(dw);
     DYN_CUDA(cudaMemcpyAsync(d->query_buf, queries, (size_t)n * sizeof(dyn_query_record), cudaMemcpyHostToDevice, s));
-    const size_t warp_smem = 4u * sizeof(QueryTeam<1u>), block_smem = sizeof(QueryTeam<4u>);
-    DYN_CUDA(cudaFuncSetAttribute(k_scene_query<1u>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)warp_smem));
-    DYN_CUDA(cudaFuncSetAttribute(k_scene_query<4u>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem));
-    const uint32_t blocks = std::min<uint32_t>(n, d->sms * 4u);
+    const uint32_t blocks = std::min<uint32_t>(n, d->sms * kBlockQueriesPerSm);
     uint32_t to_blocks = n;
     if (n > d->sms * kBlockQueriesPerSm) {  // a warp each, then a block for those the warps hand on
         k_scene_query<1u><<<std::min<uint32_t>(div_up(n, 4u), d->sms * 4u), kQueryThreads, warp_smem, s>>>(
