@@ -95,7 +95,7 @@ __device__ __forceinline__ JointSide load_joint(const DeviceWorld& w, uint32_t a
 __device__ __forceinline__ f3 from_partner(f3 v) {
     return mk3(__shfl_xor_sync(0xFFFFFFFFu, v.x, 1), __shfl_xor_sync(0xFFFFFFFFu, v.y, 1), __shfl_xor_sync(0xFFFFFFFFu, v.z, 1));
 }
-// This side's half of pair_impulse: the first body takes -j, the second +j.
+// This side's half of a pair impulse: the first body takes -j, the second +j.
 __device__ __forceinline__ void side_impulse(const JointSide& s, uint32_t side, f3 j, f3* v, f3* av) {
     const f3 dv = j * s.arm.w, da = inv_inertia_world(s.ii0, s.ii1, s.rot, cross(xyz(s.arm), j));
     *v = side ? *v + dv : *v - dv;

@@ -777,161 +777,10 @@ struct EpaOut {
     float depth;
 };
 
-// convex.wgsl:286-437. The polytope lives in the calling thread's local memory.
-__device__ EpaOut epa_tetrahedron(const DeviceWorld& w, const WShape& first, const WShape& second, const SPt* simplex) {
-    f3 poly[64];
-    uint8_t fa[128], fb[128], fcv[128];  // polytope indices are below 64
-    f3 fn[128];
-    uint8_t vis[128];
-    uint8_t na[64], nb[64], nc[64];
-    f3 nn[64];
-    EpaOut invalid{false, mk3(0.0f, 1.0f, 0.0f), 0.0f};
-    for (uint32_t i = 0; i < 4; ++i) poly[i] = simplex[i].w;
-    uint32_t vc = 4;
-    uint32_t fcount = 0;
-    const uint32_t tet[4][3] = {{0, 1, 2}, {0, 2, 3}, {0, 3, 1}, {1, 3, 2}};
-    for (uint32_t i = 0; i < 4; ++i) {
-        uint32_t a = tet[i][0], b = tet[i][1], c = tet[i][2];
-        f3 normal = cross(poly[b] - poly[a], poly[c] - poly[a]);
-        float ln = length(normal);
-        if (ln < 1e-10f) return invalid;
-        f3 unit = normal / ln;
-        f3 centroid = (poly[a] + poly[b] + poly[c]) * (1.0f / 3.0f);
-        fa[fcount] = a;
-        fb[fcount] = b;
-        fcv[fcount] = c;
-        fn[fcount] = dot(unit, centroid) > 0.0f ? -unit : unit;
-        fcount += 1;
-    }
-    float best_dist = 0.0f;
-    uint32_t best = 0;
-    for (uint32_t iter = 0; iter < 32u; ++iter) {
-        best_dist = 3.402823466e38f;
-        best = 0;
-        for (uint32_t i = 0; i < fcount; ++i) {
-            float dist = dot(fn[i], poly[fa[i]]);
-            if (dist < best_dist && length(fn[i]) > 0.5f) {
-                best_dist = dist;
-                best = i;
-            }
-        }
-        f3 probe = support_pair(w, first, second, fn[best]).w;
-        float gain = dot(probe, fn[best]) - best_dist;
-        if (gain < 1e-4f) break;
-        if (vc >= 64u) break;
-        poly[vc] = probe;
-        vc += 1;
-        uint32_t vcount = 0;
-        for (uint32_t i = 0; i < fcount; ++i) {
-            if (dot(fn[i], probe - poly[fa[i]]) > 1e-6f) {
-                vis[vcount] = i;
-                vcount += 1;
-            }
-        }
-        uint32_t ncount = 0;
-        for (uint32_t i = 0; i < vcount; ++i) {
-            uint32_t f = vis[i];
-            uint32_t ea[3] = {fa[f], fb[f], fcv[f]};
-            uint32_t eb[3] = {fb[f], fcv[f], fa[f]};
-            for (uint32_t e = 0; e < 3; ++e) {
-                uint32_t start = ea[e], end = eb[e];
-                bool shared = false;
-                for (uint32_t j = 0; j < vcount; ++j) {
-                    if (j == i) continue;
-                    uint32_t o = vis[j];
-                    if ((fa[o] == end && fb[o] == start) || (fb[o] == end && fcv[o] == start) || (fcv[o] == end && fa[o] == start)) {
-                        shared = true;
-                    }
-                }
-                if (!shared && ncount < 64u) {
-                    uint32_t apex = vc - 1u;
-                    f3 normal = cross(poly[end] - poly[apex], poly[start] - poly[apex]);
-                    float ln = length(normal);
-                    if (ln > 1e-10f) {
-                        f3 unit = normal / ln;
-                        f3 centroid = (poly[apex] + poly[start] + poly[end]) * (1.0f / 3.0f);
-                        na[ncount] = apex;
-                        nb[ncount] = start;
-                        nc[ncount] = end;
-                        nn[ncount] = dot(unit, centroid) > 0.0f ? -unit : unit;
-                        ncount += 1;
-                    }
-                }
-            }
-        }
-        uint32_t write = 0, seen = 0;
-        for (uint32_t i = 0; i < fcount; ++i) {
-            if (seen < vcount && vis[seen] == i) {
-                seen += 1;
-                continue;
-            }
-            fa[write] = fa[i];
-            fb[write] = fb[i];
-            fcv[write] = fcv[i];
-            fn[write] = fn[i];
-            write += 1;
-        }
-        fcount = write;
-        if (fcount + ncount > 128u) break;
-        for (uint32_t i = 0; i < ncount; ++i) {
-            fa[fcount] = na[i];
-            fb[fcount] = nb[i];
-            fcv[fcount] = nc[i];
-            fn[fcount] = nn[i];
-            fcount += 1;
-        }
-    }
-    best_dist = 3.402823466e38f;
-    for (uint32_t i = 0; i < fcount; ++i) {
-        float dist = dot(fn[i], poly[fa[i]]);
-        if (dist < best_dist && length(fn[i]) > 0.5f) {
-            best_dist = dist;
-            best = i;
-        }
-    }
-    EpaOut r;
-    r.valid = best_dist < 3.402823466e38f;
-    r.normal = fn[best];
-    r.depth = best_dist;
-    return r;
-}
-
 __device__ __forceinline__ float support_projection_depth(const DeviceWorld& w, const WShape& f, const WShape& s, f3 direction) {
     f3 n = normalize(direction);
     return dot(support(w, f, n) - support(w, s, -n), n);
 }
-// convex.wgsl:532-582
-// With stop_at_separation the probe returns as soon as one direction shows no overlap (depth <= 0):
-// the caller then only needs to know that the minimum is not positive, and the minimum over all
-// directions is unchanged whenever it is positive.
-__device__ EpaOut penetration_probe(const DeviceWorld& w, const WShape& first, const WShape& second, const SPt* simplex,
-                                    uint32_t count, bool stop_at_separation = false) {
-    EpaOut best{false, mk3(0.0f, 1.0f, 0.0f), 3.402823466e38f};
-    f3 probed[16];
-    uint32_t pc = 0;
-    for (uint32_t i = 0; i < count; ++i)
-        for (uint32_t j = i + 1; j < count; ++j)
-            for (uint32_t k = j + 1; k < count; ++k) {
-                f3 normal = cross(simplex[j].w - simplex[i].w, simplex[k].w - simplex[i].w);
-                if (length(normal) > 1e-8f && pc < 16u) probed[pc++] = normal;
-            }
-    f3 cdir = second.center - first.center;
-    if (length(cdir) > 1e-8f && pc < 16u) probed[pc++] = cdir;
-    const float ax[6][3] = {{1, 0, 0}, {-1, 0, 0}, {0, 1, 0}, {0, -1, 0}, {0, 0, 1}, {0, 0, -1}};
-    for (uint32_t i = 0; i < 6; ++i)
-        if (pc < 16u) probed[pc++] = mk3(ax[i][0], ax[i][1], ax[i][2]);
-    for (uint32_t i = 0; i < pc; ++i) {
-        float depth = support_projection_depth(w, first, second, probed[i]);
-        if (depth < best.depth) {
-            best.depth = depth;
-            best.normal = normalize(probed[i]);
-        }
-        if (stop_at_separation && depth <= 0.0f) break;
-    }
-    best.valid = best.depth < 3.402823466e38f;
-    return best;
-}
-
 // GJK's fixed points. The reference's search either ends within a dozen iterations or, for about one
 // pair in five that reach it, meets a simplex that an iteration turns into itself: the reduction drops
 // the newest point and the support point that replaces it is that point again. An iteration depends
@@ -951,7 +800,7 @@ __device__ __forceinline__ bool gjk_repeats(const float* lam, uint32_t count, f3
            __float_as_uint(newest.z) == __float_as_uint(support_point.z);
 }
 
-// ---- the convex path in three phases (results identical to convex_hit) ----
+// ---- the convex path in three phases (results identical to the reference's convex_hit) ----
 //
 // Phase 1, one thread per pair: GJK (convex.wgsl:464-521) and, for separated shapes, the
 // penetration probe that may still report overlap (convex.wgsl:588-600). Phase 2, one warp per
@@ -1047,18 +896,6 @@ __device__ GjkOut gjk_phase(const DeviceWorld& w, const WShape& first, const WSh
         cl = simplex_closest(o.s, o.count);
     }
     return o;
-}
-
-// convex.wgsl:588-600 for a separated GJK result.
-__device__ Hit separated_hit(const DeviceWorld& w, const WShape& first, const WShape& second, const GjkOut& g) {
-    EpaOut probe = penetration_probe(w, first, second, g.s, g.count, true);
-    if (probe.depth > 0.0f) {
-        f3 normal = probe.normal;
-        if (dot(normal, second.center - first.center) < 0.0f) normal = -normal;
-        return Hit{-probe.depth, (g.pa + g.pb) * 0.5f, normal};
-    }
-    if (g.dist > 0.0f) return Hit{g.dist, (g.pa + g.pb) * 0.5f, g.normal};
-    return Hit{3.402823466e38f, s3(0.0f), s3(0.0f)};
 }
 
 // ---- warp-cooperative pieces ----

@@ -1137,7 +1137,7 @@ __device__ __forceinline__ void gjk_separated(const Lanes<kGjkLanes>& L, const D
 // The same machine with one lane per pair, for batches that fill the chip: fewer instructions per
 // pair than a group spends (every lane of a group repeats the rotations and the tests), but a trip
 // takes the union of a warp's states and candidates. Each state does the same arithmetic, in the same
-// order, as gjk_phase followed by separated_hit (narrow.cuh).
+// order, as gjk_phase (narrow.cuh) followed by the separated pair's test (convex.wgsl:588-600).
 struct GjkLane {
     uint32_t state, index, count, iter;
     float tiny, margin, dist;
@@ -1379,9 +1379,9 @@ __global__ void __launch_bounds__(kGjkThreads, 6) k_convex_gjk_lanes(DeviceWorld
     }
 }
 
-// convex.wgsl:532-582 (penetration_probe) then separated_hit (:588-600) for the pairs GJK left
+// convex.wgsl:532-582 (penetration_probe) then the separated pair's hit (:588-600) for the pairs GJK left
 // separated: the simplex triples, the centre axis and the six axes in order, stopping at the first
-// direction with no overlap (the minimum is then not positive, which is all separated_hit asks);
+// direction with no overlap (the minimum is then not positive, which is all that test asks);
 // when every direction overlaps, the first minimum gives the penetration. One thread per pair.
 __global__ void __launch_bounds__(128) k_convex_probe(DeviceWorld w, dyn_step_params p) {
     const uint32_t count = min(w.ctl[CTL_PROBES], w.p_cap);
@@ -1890,12 +1890,6 @@ __device__ __forceinline__ void make_tangents(f3 n, f3* t1, f3* t2) {
     *t2 = cross(n, *t1);
 }
 __device__ __forceinline__ f3 arm(const DBody& b, f3 local) { return quat_rotate(b.orientation, local) + b.position; }
-__device__ __forceinline__ void pair_impulse(DBody* a, DBody* b, f3 pa, f3 pb, f3 j) {
-    a->velocity = a->velocity - j * a->inverse_mass;
-    a->angular_velocity = a->angular_velocity - dbody_iinv(*a, cross(pa - dbody_com(*a), j));
-    b->velocity = b->velocity + j * b->inverse_mass;
-    b->angular_velocity = b->angular_velocity + dbody_iinv(*b, cross(pb - dbody_com(*b), j));
-}
 __device__ __forceinline__ float momentum_mass(const DBody& a, const DBody& b, f3 pa, f3 pb, f3 axis) {
     f3 ra = pa - dbody_com(a), rb = pb - dbody_com(b);
     f3 rax = cross(ra, axis), rbx = cross(rb, axis);
