@@ -2472,4 +2472,32 @@ uint32_t orc_narrowphase_pair(const OracleWorld* w, uint32_t a, uint32_t b, dyn_
     return narrowphase_pair(*w, a, b, out) ? 1u : 0u;
 }
 
+// The GJK walks of n collider pairs at the current states, for the library's early end on a repeat.
+// out: walks that took all 24 iterations, those of them that met a repeat, and those of these whose
+// simplex at the end is not, bit for bit, the one after the repeat (a walk that ends early after a
+// repeat counts there too).
+void orc_gjk_walks(const OracleWorld* w, const uint32_t* major, const uint32_t* minor, uint32_t n, uint32_t* out) {
+    uint32_t full = 0, repeated = 0, wrong = 0;
+#pragma omp parallel for schedule(dynamic, 256) reduction(+ : full, repeated, wrong)
+    for (uint32_t i = 0; i < n; ++i) {
+        Body a = body_at(*w, w->owners[major[i]]), b = body_at(*w, w->owners[minor[i]]);
+        const dyn_collider_record &ca = w->colliders[major[i]], &cb = w->colliders[minor[i]];
+        if (shape_world_geometry(ca.kind) || shape_world_geometry(cb.kind)) continue;
+        GjkWatch watch;
+        SimplexPoint simplex[4];
+        uint32_t count = 0;
+        convex_closest(w->shapes, world_collider(a.position, a.orientation, ca), world_collider(b.position, b.orientation, cb),
+                       simplex, &count, &watch);
+        full += watch.iterations == 24u;
+        if (watch.repeat == 24u) continue;
+        repeated += watch.iterations == 24u;
+        bool same = watch.iterations == 24u && count == watch.count;
+        for (uint32_t k = 0; same && k < count; ++k) same = std::memcmp(&simplex[k], &watch.simplex[k], sizeof(SimplexPoint)) == 0;
+        wrong += !same;
+    }
+    out[0] = full;
+    out[1] = repeated;
+    out[2] = wrong;
+}
+
 }  // extern "C"

@@ -197,6 +197,17 @@ class OracleWorld:
         L.orc_query(self._h, _p(q), len(q), _p(hits))
         return q, hits[:bound]
 
+    def gjk_walks(self, major, minor) -> tuple[int, int, int]:
+        """Of the pairs' GJK walks: those of all 24 iterations, those of them that met a repeated simplex, and
+        those of these that did not keep it to the end."""
+        major, minor = np.ascontiguousarray(major, np.uint32), np.ascontiguousarray(minor, np.uint32)
+        out = np.zeros(3, np.uint32)
+        L = lib()
+        L.orc_gjk_walks.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint32, ctypes.c_void_p]
+        L.orc_gjk_walks.restype = None
+        L.orc_gjk_walks(self._h, _p(major), _p(minor), len(major), _p(out))
+        return tuple(int(x) for x in out)
+
     def resting(self) -> np.ndarray:
         """The frozen contacts: first id, its generation, second id, its generation, collider a, collider b."""
         L = lib()

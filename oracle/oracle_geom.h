@@ -9,6 +9,8 @@
 // heightfields) and hulls above 4,096 vertices (BVH support) are not restated.
 #pragma once
 
+#include <cstring>
+
 #include <vector>
 
 #include "dynamis_abi.h"
@@ -1075,9 +1077,17 @@ struct ConvexClosest {
     bool penetrating;
 };
 
+// What a walk of convex_closest did, for the check of the library's early end (orc_gjk_walks): the
+// iteration it first met a repeat on (the reduction drops the newest point and the support point that
+// replaces it equals that one bit for bit; 24: none), the simplex after it, and the iterations taken.
+struct GjkWatch {
+    uint32_t repeat = 24u, iterations = 0u, count = 0u;
+    SimplexPoint simplex[4];
+};
+
 // convex.wgsl:464-521
 inline ConvexClosest convex_closest(const Shapes& sh, const WorldShape& first, const WorldShape& second,
-                                    SimplexPoint* out_simplex, uint32_t* out_count) {
+                                    SimplexPoint* out_simplex, uint32_t* out_count, GjkWatch* watch = nullptr) {
     SimplexPoint simplex[4];
     uint32_t count = 0;
     ConvexClosest result;
@@ -1113,6 +1123,8 @@ inline ConvexClosest convex_closest(const Shapes& sh, const WorldShape& first, c
             if (result.distance > 1e-6f) result.normal = sign_normalize(closest.point_b - closest.point_a);
             break;
         }
+        bool repeats = count >= 2u && std::memcmp(&simplex[count - 1u].w, &sp.w, sizeof(V3)) == 0;
+        for (uint32_t i = 0; i < count; ++i) repeats = repeats && (closest.lambdas[i] > 1e-6f) == (i + 1u < count);
         count = simplex_reduce(simplex, closest.lambdas);
         if (simplex_holds(simplex, count, sp.w, shape_scale(second))) {
             result.distance = length(closest.v);
@@ -1123,6 +1135,14 @@ inline ConvexClosest convex_closest(const Shapes& sh, const WorldShape& first, c
         }
         simplex[count] = sp;
         count += 1;
+        if (watch) {
+            watch->iterations = iter + 1u;
+            if (repeats && watch->repeat == 24u) {
+                watch->repeat = iter;
+                watch->count = count;
+                for (uint32_t i = 0; i < count; ++i) watch->simplex[i] = simplex[i];
+            }
+        }
         closest = simplex_closest(simplex, count);
     }
     for (uint32_t i = 0; i < 4; ++i) out_simplex[i] = simplex[i];

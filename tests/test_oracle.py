@@ -260,3 +260,27 @@ def test_islands_are_minimum_rows_of_touching_groups():
     o.step(DT)
     assert list(o.islands()) == [0, 0, 0, 3, 3]
     assert o.counters()[R.COUNTER["ISLANDS"]] == 2
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_a_repeated_gjk_simplex_is_kept_to_the_iteration_limit(seed):
+    """The reference's GJK runs to 24 iterations on some pairs. The library ends a walk whose reduction
+    drops the newest point and gets it back bit for bit; here the whole walk is run after such a repeat
+    and the simplex must come out the same. No walk reaches the limit in another way."""
+    rng = np.random.default_rng(seed)
+    scene = scenes.mixed_pile(7, seed=seed)
+    n = len(scene.bodies) - 1
+    # every second pose close to another body's, over distances from deep overlap to clear separation
+    scene.bodies["position"][:n] = rng.uniform(-2.0, 2.0, (n, 3)) * rng.choice([0.3, 1.0, 3.0], (n, 1))
+    capsules = rng.random(n) < 0.3
+    scene.colliders["shape"][:n][capsules] = rng.choice([R.SHAPE_CAPSULE, R.SHAPE_CYLINDER], int(capsules.sum()))
+    scene.colliders["radius"][:n][capsules] = rng.uniform(0.1, 0.5, int(capsules.sum()))
+    scene.colliders["half_height"][:n][capsules] = rng.uniform(0.1, 0.6, int(capsules.sum()))
+    w = World()
+    scene.build(w)
+    o = O.oracle_from_world(w, DT)
+    major, minor = np.triu_indices(n, 1)
+    full, repeated, wrong = o.gjk_walks(major, minor)
+    assert len(major) > 50000 and full > 500
+    assert repeated == full and wrong == 0
+    w.close()
